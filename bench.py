@@ -110,10 +110,10 @@ FORMS = {"pcg": "plain FP64 Jacobi-PCG",
 
 
 FORMS["ml"] = ("FP64 flexible CG preconditioned by one aggregation-multigrid V-cycle on D^-1-scaled FP32 levels "
-               "(pairwise aggregation, 3 passes per level, dense coarsest level; meshes of >= 2^20 cells: "
+               "(pairwise aggregation, dense coarsest level; meshes of >= 65 536 cells: smoothed aggregation, "
                "standalone full-occupancy kernels, Chebyshev degree 2; smaller: one persistent kernel, degree 3)")
 KERNELS = {"pcg": "k_pcg (persistent Jacobi-PCG)", "fcg": "k_fcg (persistent two-level flexible CG)",
-           "ml": "multilevel flexible CG (k_mlk_* standalone kernels on >= 2^20 cells, else persistent k_mlcg): "
+           "ml": "multilevel flexible CG (k_mlk_* standalone kernels on >= 65 536 cells, else persistent k_mlcg): "
                  "whole pressure solve"}
 
 

@@ -164,7 +164,7 @@ int run_ml(double rtol, double atol, int maxit, int* reason, int* its, double* r
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, g_ctx.device);
     if (g_ctx.ml->setup(g_ctx.n, g_ctx.WA, g_ctx.hcol.data(), g_ctx.hval.data(), g_ctx.col, g_ctx.val, nullsp != 0, 0,
-                        0, 0.0, sms, g_ctx.bar, g_ctx.status, g_ctx.dout)) {
+                        0, 0.0, sms, g_ctx.bar, g_ctx.status, g_ctx.dout, 0, 0)) {
       delete g_ctx.ml;
       g_ctx.ml = nullptr;
       return -26;

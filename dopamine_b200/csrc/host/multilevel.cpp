@@ -10,8 +10,8 @@ namespace {
 struct Csr {
   int n = 0;
   std::vector<int64_t> off;
-  std::vector<int> col;
-  std::vector<double> val;
+  Raw<int> col;
+  Raw<double> val;
 };
 
 // Rows are independent: counted in parallel, then filled in parallel at their prefix offsets.
@@ -195,15 +195,19 @@ Csr galerkin(const Csr& A, const std::vector<int>& agg, int na) {
   return C;
 }
 
-// Largest eigenvalue of D^-1 A by 30 power steps from a fixed start vector.  The norms are summed
+// Largest eigenvalue of D^-1 A by `steps` power steps from a fixed start vector.  The norms are summed
 // over fixed chunks of rows, then the chunks in order: the same value on any number of threads.
-double lambda_max(const Csr& A, const std::vector<double>& dinv) {
+// noise: a hashed start vector; the smooth default start is close to the operator's constant mode and
+// takes its 30 steps to leave it.
+double lambda_max(const Csr& A, const std::vector<double>& dinv, int steps = 30, bool noise = false) {
   constexpr int CH = 16384;
   const int n = A.n, nch = (n + CH - 1) / CH;
   std::vector<double> v(n), w(n), pv(nch), pw(nch);
-  for (int i = 0; i < n; ++i) v[i] = 1.0 + 0.5 * std::sin(0.7 * i + 0.3);
+#pragma omp parallel for schedule(static)
+  for (int i = 0; i < n; ++i)
+    v[i] = noise ? (double)((uint32_t)i * 2654435761u >> 8) / 8388608.0 - 1.0 : 1.0 + 0.5 * std::sin(0.7 * i + 0.3);
   double lam = 0.0;
-  for (int it = 0; it < 30; ++it) {
+  for (int it = 0; it < steps; ++it) {
 #pragma omp parallel for schedule(static)
     for (int c = 0; c < nch; ++c) {
       double nv = 0.0, nw = 0.0;
@@ -229,16 +233,21 @@ double lambda_max(const Csr& A, const std::vector<double>& dinv) {
   return lam;
 }
 
+// Lower Cholesky factor in place; each entry is one inner product over a fixed range, so the
+// result does not depend on the thread count.
 bool cholesky_lower(std::vector<double>& a, int n) {
   for (int j = 0; j < n; ++j) {
-    double d = a[(size_t)j * n + j];
-    for (int k = 0; k < j; ++k) d -= a[(size_t)j * n + k] * a[(size_t)j * n + k];
+    const double* rj = &a[(size_t)j * n];
+    double d = rj[j];
+    for (int k = 0; k < j; ++k) d -= rj[k] * rj[k];
     if (!(d > 0.0)) return false;
     d = std::sqrt(d);
     a[(size_t)j * n + j] = d;
+#pragma omp parallel for schedule(static) if (n - j > 128)
     for (int i = j + 1; i < n; ++i) {
-      double s = a[(size_t)i * n + j];
-      for (int k = 0; k < j; ++k) s -= a[(size_t)i * n + k] * a[(size_t)j * n + k];
+      const double* ri = &a[(size_t)i * n];
+      double s = ri[j];
+      for (int k = 0; k < j; ++k) s -= ri[k] * rj[k];
       a[(size_t)i * n + j] = s / d;
     }
   }
@@ -259,21 +268,29 @@ int dense_inverse(const Csr& A, bool nullsp, std::vector<float>& out) {
     for (auto& x : a) x += s;
   }
   if (!cholesky_lower(a, n)) return -4;
-  out.assign((size_t)n * n, 0.0f);
-  std::vector<double> y(n);
-  for (int c = 0; c < n; ++c) {  // column c of the inverse: L L^T y = e_c
-    for (int i = 0; i < n; ++i) {
+  // rows of yt: the columns of L^-1 (L y = e_c, zero above c), then A^-1 = L^-T L^-1 by inner
+  // products of those rows
+  std::vector<double> yt((size_t)n * n, 0.0);
+#pragma omp parallel for schedule(dynamic, 8)
+  for (int c = 0; c < n; ++c) {
+    double* y = &yt[(size_t)c * n];
+    for (int i = c; i < n; ++i) {
+      const double* ri = &a[(size_t)i * n];
       double s = i == c ? 1.0 : 0.0;
-      for (int k = 0; k < i; ++k) s -= a[(size_t)i * n + k] * y[k];
-      y[i] = s / a[(size_t)i * n + i];
+      for (int k = c; k < i; ++k) s -= ri[k] * y[k];
+      y[i] = s / ri[i];
     }
-    for (int i = n - 1; i >= 0; --i) {
-      double s = y[i];
-      for (int k = i + 1; k < n; ++k) s -= a[(size_t)k * n + i] * y[k];
-      y[i] = s / a[(size_t)i * n + i];
-    }
-    for (int i = 0; i < n; ++i) out[(size_t)i * n + c] = (float)y[i];
   }
+  out.assign((size_t)n * n, 0.0f);
+#pragma omp parallel for schedule(dynamic, 8)
+  for (int i = 0; i < n; ++i)
+    for (int j = 0; j <= i; ++j) {
+      const double *yi = &yt[(size_t)i * n], *yj = &yt[(size_t)j * n];
+      double s = 0.0;
+      for (int k = i; k < n; ++k) s += yi[k] * yj[k];
+      out[(size_t)i * n + j] = (float)s;
+      out[(size_t)j * n + i] = (float)s;
+    }
   return 0;
 }
 
@@ -363,7 +380,337 @@ MlLevel make_level(const Csr& A, const std::vector<int>& agg, int na, int& rc) {
   return L;
 }
 
+// `passes` pairwise passes on A: the aggregate of every row and the operator T^T A T.
+Csr aggregate(const Csr& A, double beta, int passes, std::vector<int>& agg_tot) {
+  Csr Ac;
+  for (int p = 0; p < passes; ++p) {
+    std::vector<int> agg;
+    const Csr& from = p == 0 ? A : Ac;
+    const int na = pairwise(from, beta, agg);
+    Csr next = galerkin(from, agg, na);
+    if (p == 0) agg_tot = agg;
+    else {
+#pragma omp parallel for schedule(static)
+      for (int i = 0; i < A.n; ++i) agg_tot[i] = agg[agg_tot[i]];
+    }
+    Ac = std::move(next);
+  }
+  return Ac;
+}
+
+// Smoothed prolongation by rows: row i of (I - w D^-1 A_F) T, columns in order of first appearance.
+void smooth_prolongation(const Csr& A, const std::vector<double>& dinv, const std::vector<int>& agg, double w,
+                         double theta, Raw<int>& off, Raw<SaEntry>& ent) {
+  // one row into c / v; returns its entries
+  auto row = [&](int i, std::vector<int>& c, std::vector<double>& v) {
+    double mx = 0.0, dg = 0.0;
+    for (int64_t k = A.off[i]; k < A.off[i + 1]; ++k)
+      if (A.col[k] != i) mx = std::max(mx, -A.val[k]);
+    for (int64_t k = A.off[i]; k < A.off[i + 1]; ++k)
+      if (A.col[k] == i || -A.val[k] < theta * mx) dg += A.val[k];
+    c.assign(1, agg[i]);
+    v.assign(1, 1.0 - w * dg * dinv[i]);
+    for (int64_t k = A.off[i]; k < A.off[i + 1]; ++k) {
+      const int j = A.col[k];
+      if (j == i || -A.val[k] < theta * mx) continue;
+      size_t t = 0;
+      while (t < c.size() && c[t] != agg[j]) ++t;
+      if (t == c.size()) {
+        c.push_back(agg[j]);
+        v.push_back(0.0);
+      }
+      v[t] -= w * A.val[k] * dinv[i];
+    }
+    return (int)c.size();
+  };
+  off.resize((size_t)A.n + 1);
+  off[0] = 0;
+#pragma omp parallel
+  {
+    std::vector<int> c;
+    std::vector<double> v;
+#pragma omp for schedule(static)
+    for (int i = 0; i < A.n; ++i) off[i + 1] = row(i, c, v);
+  }
+  for (int i = 0; i < A.n; ++i) off[i + 1] += off[i];
+  ent.resize(off[A.n]);
+#pragma omp parallel
+  {
+    std::vector<int> c;
+    std::vector<double> v;
+#pragma omp for schedule(static)
+    for (int i = 0; i < A.n; ++i) {
+      const int m = row(i, c, v);
+      for (int k = 0; k < m; ++k) ent[off[i] + k] = {c[k], (float)v[k]};
+    }
+  }
+}
+
+// P^T by rows (fine rows ascending in each): slots taken concurrently, then every row sorted, so
+// the result is the same on any thread count.
+void transpose(int n, int na, const Raw<int>& off, const Raw<SaEntry>& ent, Raw<int>& toff, Raw<SaEntry>& tent) {
+  std::vector<int> cnt(na, 0);
+#pragma omp parallel for schedule(static)
+  for (int k = 0; k < off[n]; ++k) {
+#pragma omp atomic
+    cnt[ent[k].col]++;
+  }
+  toff.resize((size_t)na + 1);
+  toff[0] = 0;
+  for (int a = 0; a < na; ++a) {
+    toff[a + 1] = toff[a] + cnt[a];
+    cnt[a] = toff[a];
+  }
+  tent.resize(off[n]);
+#pragma omp parallel for schedule(static)
+  for (int i = 0; i < n; ++i)
+    for (int k = off[i]; k < off[i + 1]; ++k) {
+      int slot;
+#pragma omp atomic capture
+      slot = cnt[ent[k].col]++;
+      tent[slot] = {i, ent[k].val};
+    }
+#pragma omp parallel for schedule(static)
+  for (int a = 0; a < na; ++a)
+    std::sort(tent.begin() + toff[a], tent.begin() + toff[a + 1],
+              [](const SaEntry& x, const SaEntry& y) { return x.col < y.col; });
+}
+
+// Rows formed one by one by fn(i, add), add(column, value) accumulating the row's entries: a chunk
+// of rows per thread at a time, each row's columns sorted.  Every row is formed in a fixed order.
+template <class Fn>
+Csr accumulate_rows(int n, int ncol, Fn fn) {
+  Csr C;
+  C.n = n;
+  const int CH = std::max(16, std::min(4096, n / 512));
+  const int nch = (n + CH - 1) / CH;
+  std::vector<Raw<int>> cc(nch);
+  std::vector<Raw<double>> vv(nch);
+  C.off.assign((size_t)n + 1, 0);
+#pragma omp parallel
+  {
+    std::vector<int> pos(ncol, -1), cols, order;
+    std::vector<double> vals;
+    auto add = [&](int c, double v) {
+      if (pos[c] < 0) {
+        pos[c] = (int)cols.size();
+        cols.push_back(c);
+        vals.push_back(0.0);
+      }
+      vals[pos[c]] += v;
+    };
+#pragma omp for schedule(dynamic, 1)
+    for (int ch = 0; ch < nch; ++ch) {
+      const int i1 = std::min(n, (ch + 1) * CH);
+      for (int i = ch * CH; i < i1; ++i) {
+        cols.clear();
+        vals.clear();
+        fn(i, add);
+        order = cols;
+        std::sort(order.begin(), order.end());
+        for (int c : order) {
+          cc[ch].push_back(c);
+          vv[ch].push_back(vals[pos[c]]);
+        }
+        for (int c : cols) pos[c] = -1;
+        C.off[i + 1] = (int64_t)cols.size();
+      }
+    }
+  }
+  for (int i = 0; i < n; ++i) C.off[i + 1] += C.off[i];
+  C.col.resize(C.off[n]);
+  C.val.resize(C.off[n]);
+#pragma omp parallel for schedule(dynamic, 1)
+  for (int ch = 0; ch < nch; ++ch) {
+    std::copy(cc[ch].begin(), cc[ch].end(), C.col.begin() + C.off[(size_t)ch * CH]);
+    std::copy(vv[ch].begin(), vv[ch].end(), C.val.begin() + C.off[(size_t)ch * CH]);
+  }
+  return C;
+}
+
+// P^T A P.  Short rows of A (the finest level): in one product per coarse row, so that A P, the
+// largest array, is never stored; long ones: P^T (A P), a quarter of the multiplications.
+Csr galerkin_smoothed(const Csr& A, int na, const Raw<int>& poff, const Raw<SaEntry>& pent, const Raw<int>& roff,
+                      const Raw<SaEntry>& rent) {
+  if (A.off[A.n] < 16 * (int64_t)A.n)
+    return accumulate_rows(na, na, [&](int a, auto& add) {
+      for (int m = roff[a]; m < roff[a + 1]; ++m) {
+        const int i = rent[m].col;
+        for (int64_t k = A.off[i]; k < A.off[i + 1]; ++k) {
+          const double w = (double)rent[m].val * A.val[k];
+          const int j = A.col[k];
+          for (int q = poff[j]; q < poff[j + 1]; ++q) add(pent[q].col, w * (double)pent[q].val);
+        }
+      }
+    });
+  const Csr AP = accumulate_rows(A.n, na, [&](int i, auto& add) {
+    for (int64_t k = A.off[i]; k < A.off[i + 1]; ++k) {
+      const int j = A.col[k];
+      for (int q = poff[j]; q < poff[j + 1]; ++q) add(pent[q].col, A.val[k] * (double)pent[q].val);
+    }
+  });
+  return accumulate_rows(na, na, [&](int a, auto& add) {
+    for (int m = roff[a]; m < roff[a + 1]; ++m) {
+      const int i = rent[m].col;
+      for (int64_t k = AP.off[i]; k < AP.off[i + 1]; ++k) add(AP.col[k], (double)rent[m].val * AP.val[k]);
+    }
+  });
+}
+
+// The smoother's scaled off-diagonal form of A: ELL (finest level) or compressed rows.
+int scaled_rows(const Csr& A, const std::vector<double>& dinv, bool ell, bool half, SaLevel& L) {
+  const int n = A.n;
+  L.n = n;
+  L.g.resize(n);
+  L.diag.resize(n);
+  L.dinv.resize(n);
+  if (ell) {
+    L.Wo = 1;
+    for (int i = 0; i < n; ++i) L.Wo = std::max<int>(L.Wo, (int)(A.off[i + 1] - A.off[i]) - 1);
+    L.ocol.resize((size_t)L.Wo * n);
+    if (half) L.sv16.resize((size_t)L.Wo * n);
+    else L.sv32.resize((size_t)L.Wo * n);
+  } else {
+    if (A.off[n] - n > 2000000000LL) return -6;
+    L.off.resize((size_t)n + 1);
+    for (int i = 0; i <= n; ++i) L.off[i] = (int)(A.off[i] - i);  // one diagonal entry per row left out
+    L.ent.resize(L.off[n]);
+  }
+#pragma omp parallel for schedule(static)
+  for (int i = 0; i < n; ++i) {
+    int s = 0;
+    double d = 1.0;
+    for (int64_t k = A.off[i]; k < A.off[i + 1]; ++k) {
+      if (A.col[k] == i) continue;
+      const double sij = A.val[k] * dinv[i];
+      if (ell) {
+        const size_t e = (size_t)s * n + i;
+        L.ocol[e] = A.col[k];
+        if (half) {
+          L.sv16[e] = half_bits(sij);
+          d += sij - half_value(L.sv16[e]);
+        } else {
+          L.sv32[e] = (float)sij;
+          d += sij - (double)L.sv32[e];
+        }
+      } else {
+        const size_t e = (size_t)L.off[i] + s;
+        L.ent[e] = {A.col[k], (float)sij};
+        d += sij - (double)L.ent[e].val;
+      }
+      ++s;
+    }
+    if (ell)
+      for (; s < L.Wo; ++s) {
+        const size_t e = (size_t)s * n + i;
+        L.ocol[e] = i;
+        if (half) L.sv16[e] = 0;
+        else L.sv32[e] = 0.0f;
+      }
+    L.g[i] = (float)d;
+    L.diag[i] = (float)(1.0 / dinv[i]);
+    L.dinv[i] = (float)dinv[i];
+  }
+  return 0;
+}
+
 }  // namespace
+
+int build_smoothed_multilevel(int n, int WA, const int* A_col, const double* A_val, bool nullsp, int passes,
+                              double beta, double oc, bool half, int ncoarse, SaMultilevel& M) {
+  constexpr double OMEGA = 1.5, THETA = 0.25;
+  if (n < 1 || WA < 1 || WA > 64 || passes < 1 || ncoarse < 1) return -1;
+  M = SaMultilevel{};
+  Csr A = csr_from_ell(n, WA, A_col, A_val), U;  // U: the unsmoothed Galerkin operator of this level
+  for (;;) {
+    const Csr& from = M.lv.empty() ? A : U;
+    M.sizes.push_back(A.n);
+    if (A.n <= ncoarse) break;
+    if ((int)M.lv.size() >= ML_MAX_LEVELS) return -3;
+    std::vector<double> dinv(A.n, 0.0);
+    int bad = 0;
+    double bound = 0.0;
+#pragma omp parallel for schedule(static) reduction(| : bad) reduction(max : bound)
+    for (int i = 0; i < A.n; ++i) {
+      double dg = 0.0, s = 0.0;
+      int nd = 0;
+      for (int64_t k = A.off[i]; k < A.off[i + 1]; ++k) {
+        s += std::fabs(A.val[k]);
+        if (A.col[k] == i) {
+          dg = A.val[k];
+          ++nd;
+        }
+      }
+      if (!(dg > 0.0) || nd != 1) {
+        bad = 1;
+        continue;
+      }
+      dinv[i] = 1.0 / dg;
+      bound = std::max(bound, s * dinv[i]);
+    }
+    if (bad) return -5;
+    SaLevel L;
+    // The finest level's rows are diagonally dominant, where Gershgorin's bound is close (2 against
+    // 1.85-1.99 on the hex meshes); on the others (2-4 against 1.3-2) power steps, which have been
+    // seen to stop up to 15 % short of the largest eigenvalue.  Chebyshev steps on 1.1 lmax still
+    // damp up to 1.21 lmax.
+    L.lmax = M.lv.empty() ? 0.97 * bound : 1.08 * lambda_max(A, dinv, 20, true);
+    int rc = scaled_rows(A, dinv, M.lv.empty(), half, L);
+    if (rc) return rc;
+    std::vector<int> agg;
+    Csr Un = aggregate(from, beta, passes + (M.lv.empty() ? 0 : 1), agg);
+    const int na = Un.n;
+    if (na > 0.85 * A.n) return -2;
+    Csr C;
+    bool smoothed = passes >= 3;
+    if (smoothed) {
+      smooth_prolongation(A, dinv, agg, OMEGA / L.lmax, THETA, L.poff, L.pent);
+      transpose(A.n, na, L.poff, L.pent, L.roff, L.rent);
+      C = galerkin_smoothed(A, na, L.poff, L.pent, L.roff, L.rent);
+      smoothed = C.off[na] <= A.off[A.n];
+    }
+    if (!smoothed) {
+      L.oc = (float)oc;
+      L.poff.resize((size_t)A.n + 1);
+      L.pent.resize(A.n);
+      for (int i = 0; i <= A.n; ++i) L.poff[i] = i;
+      for (int i = 0; i < A.n; ++i) L.pent[i] = {agg[i], 1.0f};
+      transpose(A.n, na, L.poff, L.pent, L.roff, L.rent);
+      C = galerkin(A, agg, na);
+    }
+    L.n_next = na;
+    M.lv.push_back(std::move(L));
+    A = std::move(C);
+    U = std::move(Un);
+  }
+  M.nC = A.n;
+  return dense_inverse(A, nullsp, M.cinv);
+}
+
+bool slice_rows(int rows, const Raw<int>& off, const Raw<SaEntry>& ent, Raw<int>& soff, Raw<SaEntry>& sent) {
+  const int ns = (rows + 31) / 32;
+  soff.resize((size_t)ns + 1);
+  int64_t total = 0;
+  for (int s = 0; s < ns; ++s) {
+    int w = 0;
+    for (int i = 32 * s; i < std::min(rows, 32 * s + 32); ++i) w = std::max(w, off[i + 1] - off[i]);
+    soff[s] = (int)total;
+    total += 32 * (int64_t)w;
+    if (total > 2147483647) return false;
+  }
+  soff[ns] = (int)total;
+  sent.resize(total);
+#pragma omp parallel for schedule(static)
+  for (int s = 0; s < ns; ++s) {
+    const int w = (soff[s + 1] - soff[s]) / 32;
+    for (int r = 0; r < 32; ++r) {
+      const int i = 32 * s + r, m0 = i < rows ? off[i] : 0, mn = i < rows ? off[i + 1] - m0 : 0;
+      for (int k = 0; k < w; ++k)
+        sent[soff[s] + 32 * (int64_t)k + r] = k < mn ? ent[m0 + k] : SaEntry{mn > 0 ? ent[m0].col : 0, 0.0f};
+    }
+  }
+  return true;
+}
 
 int build_multilevel(int n, int WA, const int* A_col, const double* A_val, bool nullsp, int passes, double beta,
                      int ncoarse, int max_dense, Multilevel& M) {

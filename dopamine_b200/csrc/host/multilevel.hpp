@@ -12,9 +12,34 @@
 // (src/solver/pressure_backend_petsc.c:381-463); the Krylov stopping rule is kept identical.
 #pragma once
 #include <cstdint>
+#include <memory>
 #include <vector>
 
 namespace dpm {
+
+// Arrays that are filled in parallel right after they are sized: resize leaves them uninitialised,
+// so that their pages are first touched by the threads that fill them.
+template <class T>
+struct RawAlloc : std::allocator<T> {
+  template <class U>
+  struct rebind {
+    using other = RawAlloc<U>;
+  };
+  template <class U>
+  void construct(U*) noexcept {}
+  template <class U, class A, class... R>
+  void construct(U* p, A&& a, R&&... r) {
+    ::new ((void*)p) U(std::forward<A>(a), std::forward<R>(r)...);
+  }
+};
+template <class T>
+using Raw = std::vector<T, RawAlloc<T>>;
+
+// An entry of a compressed row as the device reads it.
+struct SaEntry {
+  int col;
+  float val;
+};
 
 constexpr int ML_MAX_LEVELS = 12;
 constexpr int ML_MAX_DEGREE = 8;
@@ -45,6 +70,50 @@ struct Multilevel {
   std::vector<int> sizes;         // rows per level, coarsest last
   std::vector<int64_t> nnz;       // non-zeros per level, coarsest last
 };
+
+// One level of the smoothed-aggregation hierarchy, which the standalone-kernel form of the solve
+// uses.  The transfer to the next level is P = (I - (omega / lmax) D^-1 A_F) T: the piecewise-
+// constant prolongation T of the same pairwise aggregates, smoothed by one Jacobi step on A_F, the
+// operator whose weak entries (-a_ij < theta max_k(-a_ik)) are lumped on the diagonal; the next
+// operator is the Galerkin product P^T A P of the stored FP32 P, so no over-correction is needed.
+// The aggregates of every level come from the unsmoothed Galerkin operators, which stay sparse.  The smoother reads
+// the operator in the scaled off-diagonal form of MlLevel: the finest level in ELL, the others
+// (about 30-40 entries per row) in compressed rows.
+struct SaLevel {
+  int n = 0, n_next = 0;
+  int Wo = 0;                            // finest level: ELL width, ocol / sv32 / sv16 as in MlLevel
+  Raw<int> ocol;
+  Raw<float> sv32;
+  Raw<unsigned short> sv16;
+  Raw<int> off;                          // other levels: off-diagonal rows, s_ij = a_ij / a_ii
+  Raw<SaEntry> ent;
+  Raw<float> g, diag, dinv;              // [n] as in MlLevel (g for the stored values in use)
+  Raw<int> poff;                         // P by rows of this level
+  Raw<SaEntry> pent;
+  Raw<int> roff;                         // P^T by rows of the next level, fine rows ascending
+  Raw<SaEntry> rent;
+  float oc = 1.0f;                       // factor of the coarse correction (1.6: unsmoothed transfer)
+  double lmax = 0.0;
+};
+
+struct SaMultilevel {
+  std::vector<SaLevel> lv;
+  int nC = 0;
+  std::vector<float> cinv;               // [nC][nC]
+  std::vector<int> sizes;
+};
+
+// A as for build_multilevel.  passes: pairwise passes of the first coarsening (deeper levels take
+// one more); with fewer than three, or where the smoothed Galerkin operator would hold more
+// entries than the level itself, the transfer stays unsmoothed with the over-correction oc.
+// half: the finest level's off-diagonals in binary16.  Coarsening stops at <= ncoarse rows.
+int build_smoothed_multilevel(int n, int WA, const int* A_col, const double* A_val, bool nullsp, int passes,
+                              double beta, double oc, bool half, int ncoarse, SaMultilevel& M);
+
+// Compressed rows to slices of 32 rows, as wide as the slice's longest row: entry k of the slice's
+// row r at soff[slice] + 32 k + r, short rows padded with (their first column, 0).  False when the
+// slices do not fit 31-bit offsets.
+bool slice_rows(int rows, const Raw<int>& off, const Raw<SaEntry>& ent, Raw<int>& soff, Raw<SaEntry>& sent);
 
 // A in padded ELL [WA][n] (padding = (own row, 0)); nullsp = the operator has the constant null
 // space.  Coarsening stops at <= ncoarse rows; returns 0, or a negative code when the coarsening

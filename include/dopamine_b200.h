@@ -152,9 +152,10 @@ typedef struct dpm_params {
    * temperature, initial Obukhov length (0 = neutral) and whether its domain mean is updated. */
   double abl_z0_m, abl_z0_h, abl_T_surface, abl_L_obukhov;
   int abl_compute_L;
-  /* DPM_PSOLVER_MULTILEVEL_FCG: Chebyshev steps per smoothing (0: 3), over-correction of the
-   * coarse correction (0: 1.6), pairwise-aggregation passes per level (0: 3; at most 3, as an
-   * aggregate of up to 3^passes rows must fit the 32 lanes of the restriction). */
+  /* DPM_PSOLVER_MULTILEVEL_FCG: Chebyshev steps per smoothing (0: 3, or 2 from 65 536 cells, where
+   * the hierarchy is smoothed aggregation), over-correction of the coarse correction of unsmoothed
+   * transfers (0: 1.6), pairwise-aggregation passes per level (0: 3; at most 3, as an aggregate of
+   * up to 3^passes rows must fit the 32 lanes of the restriction; below 3 no transfer is smoothed). */
   int p_ml_degree;
   double p_ml_overcorrect;
   int p_ml_passes;
@@ -569,8 +570,8 @@ int dpm_learn_export(dpm_solver_t* s, float* feat, unsigned* lpk, int* col, doub
 int dpm_learn_loss_grad(dpm_solver_t* s, const float* params, double* loss, float* grad);
 int dpm_download_scalars(dpm_solver_t* s, double* C);
 
-/* Aggregation hierarchy of DPM_PSOLVER_MULTILEVEL_FCG for an operator in padded ELL [width][n]
- * (host memory, no device needed): rows and non-zeros per level, coarsest last.  Returns the
+/* Unsmoothed aggregation hierarchy of DPM_PSOLVER_MULTILEVEL_FCG (the one its persistent kernel
+ * uses, below 65 536 cells) for an operator in padded ELL [width][n] (host memory, no device needed): rows and non-zeros per level, coarsest last.  Returns the
  * number of levels (<= max_levels) or a negative code. */
 int dpm_multilevel_hierarchy(int n, int width, const int* col, const double* val, int nullsp, int passes,
                              int* sizes, long long* nnz, int max_levels);
