@@ -27,6 +27,7 @@
 #include "../../../include/dopamine_b200.h"
 #include "common.cuh"
 #include "pcg.cuh"
+#include "pcg_cluster.cuh"
 #include "mlsolve.cuh"
 
 namespace {
@@ -43,6 +44,7 @@ struct Ctx {
   double *val = nullptr, *dinv = nullptr, *b = nullptr, *x = nullptr, *r = nullptr, *z = nullptr, *p0 = nullptr,
          *p1 = nullptr, *q = nullptr, *bp = nullptr, *part = nullptr, *dout = nullptr, *tot = nullptr;
   void* kernel = nullptr;
+  PcgCluster cluster;  // small systems: the solve on one cluster
   dpm::gpu::MlSolver* ml = nullptr;  // multilevel solve of the current operator (AMG names)
   int ml_nullsp = -1;
   std::vector<int> hcol;             // host copy of the operator, kept for the multilevel set-up
@@ -143,6 +145,7 @@ int build(int n, int nfaces, const int* l2g, const int* fo, const int* fnl, cons
     g_ctx.kernel = pcg_kernel_for<double>(n, g_ctx.grid, WA, &cpt);
     cudaFuncSetAttribute(g_ctx.kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 5);
   }
+  g_ctx.cluster.plan(n, WA);
   if (dalloc(&g_ctx.part, 8 * (size_t)g_ctx.grid)) return -11;
   g_ctx.n = n;
   g_ctx.nfaces = nfaces;
@@ -185,8 +188,10 @@ int run_pcg(double rtol, double atol, int maxit, int guess_zero, int* reason, in
   cudaMemsetAsync(g_ctx.bar, 0, 2 * sizeof(unsigned), g_ctx.st);
   cudaMemsetAsync(g_ctx.status, 0, 4 * sizeof(int), g_ctx.st);
   void* args[] = {&a};
-  if (cudaLaunchCooperativeKernel(g_ctx.kernel, dim3(g_ctx.grid), dim3(PCG_TPB), args, 0, g_ctx.st) != cudaSuccess)
-    return -33;
+  const cudaError_t le = g_ctx.cluster.kernel ? g_ctx.cluster.launch(a, g_ctx.st)
+                                              : cudaLaunchCooperativeKernel(g_ctx.kernel, dim3(g_ctx.grid),
+                                                                            dim3(PCG_TPB), args, 0, g_ctx.st);
+  if (le != cudaSuccess) return -33;
   int hs[4];
   double hd[4];
   cudaMemcpyAsync(hs, g_ctx.status, sizeof(hs), cudaMemcpyDeviceToHost, g_ctx.st);

@@ -32,6 +32,7 @@
 #include "../../../include/dopamine_b200.h"
 #include "common.cuh"
 #include "pcg.cuh"
+#include "pcg_cluster.cuh"
 
 namespace {
 using namespace dpm::gpu;
@@ -60,7 +61,7 @@ int scratch_address(void** ptr) {
   return 0;
 }
 
-// Every k_pcg instantiation the solve can pick (cells per thread 0..4, row width 7 or runtime):
+// Every k_pcg and k_pcg_cluster instantiation the solve can pick (row width 7 or runtime):
 // querying their attributes makes the runtime load them now rather than at a later launch.
 int preload_kernels() {
   const void* ks[] = {(const void*)k_pcg<double, 0, 7>, (const void*)k_pcg<double, 1, 7>,
@@ -73,6 +74,12 @@ int preload_kernels() {
     if (cudaFuncGetAttributes(&fa, k) != cudaSuccess) return DPM_ERR_CUDA;
     if (cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 5) != cudaSuccess) return DPM_ERR_CUDA;
   }
+  for (int cpt = 1; cpt <= PCG_CL_CPT; ++cpt)
+    for (int width : {7, 0}) {
+      cudaFuncAttributes fa;
+      const void* k = PcgCluster::pick(cpt, width);
+      if (cudaFuncGetAttributes(&fa, k) != cudaSuccess || !PcgCluster::prepare(k)) return DPM_ERR_CUDA;
+    }
   return 0;
 }
 
@@ -156,7 +163,11 @@ extern "C" int dpm_pcg_solve_noalloc(int n_cells, int row_width, const int* col,
   a.nullsp = null_space ? 1 : 0;
   a.guess_zero = 0;
   void* args[] = {&a};
-  if (cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(PCG_TPB), args, 0, st) != cudaSuccess) return DPM_ERR_CUDA;
+  PcgCluster cluster;
+  cluster.plan(n_cells, row_width);
+  const cudaError_t le = cluster.kernel ? cluster.launch(a, st)
+                                        : cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(PCG_TPB), args, 0, st);
+  if (le != cudaSuccess) return DPM_ERR_CUDA;
   int hs[4];
   double hd[4];
   if (cudaMemcpyAsync(hs, status, sizeof(hs), cudaMemcpyDeviceToHost, st) != cudaSuccess) return DPM_ERR_CUDA;

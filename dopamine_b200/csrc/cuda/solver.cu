@@ -33,6 +33,7 @@
 #include "learn.cuh"
 #include "mlsolve.cuh"
 #include "pcg.cuh"
+#include "pcg_cluster.cuh"
 #include "sampling.cuh"
 #include "sem.cuh"
 #include "scalars.cuh"
@@ -221,6 +222,7 @@ struct Solver {
   unsigned* cg_bar;
   int* cg_status;
   int cg_grid = 0;
+  PcgCluster cg_cluster;  // small meshes: the solve on one cluster (unless a poll limit is set)
   bool cg_coop = true;
   // temperature (transported when Boussinesq is on) and passive scalars, scalar-major
   double *Tb = nullptr, *gT = nullptr, *HT = nullptr, *HT0 = nullptr;
@@ -597,6 +599,7 @@ struct Solver {
         CK(cudaFuncSetAttribute(cg_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 5));
       }
     }
+    cg_cluster.plan(nc, S.WA);
     cg_part = mem.alloc<double>(8 * (size_t)cg_grid);
     {
       int rc = setup_scalars();
@@ -1594,7 +1597,8 @@ struct Solver {
     CK(cudaMemsetAsync(cg_status, 0, 4 * sizeof(int), st));
     if (spin_limit) CK(cudaMemcpyAsync(cg_status + 3, &spin_limit, sizeof(int), cudaMemcpyHostToDevice, st));
     void* args[] = {&a};
-    CK(cudaLaunchCooperativeKernel(cg_kernel, dim3(cg_grid), dim3(PCG_TPB), args, 0, st));
+    if (cg_cluster.kernel && !spin_limit) CK(cg_cluster.launch(a, st));
+    else CK(cudaLaunchCooperativeKernel(cg_kernel, dim3(cg_grid), dim3(PCG_TPB), args, 0, st));
     launches++;
     int h_st[4];
     double h_d[4];
