@@ -102,8 +102,7 @@ __device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned& gen, int* 
       if (++spins > lim) { ok = 0; atomicExch(&status[2], 1); break; }
       if (spins > 32) __nanosleep(20);
     }
-    __threadfence();
-    s_okb = ok;
+    s_okb = ok;  // the acquiring load orders what the block reads after the next barrier
   }
   __syncthreads();
   gen = gen + 1u;
@@ -156,7 +155,6 @@ __device__ __forceinline__ bool grid_reduce_gather(double (&v)[NV + NG], double*
       if (++spins > lim) { ok = 0; atomicExch(&status[2], 1); break; }
       if (spins > 32) __nanosleep(20);
     }
-    __threadfence();
     s_ok = ok && P <= 32 * RB;
     if (P > 32 * RB) atomicExch(&status[2], 2);
   }

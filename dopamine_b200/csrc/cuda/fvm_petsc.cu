@@ -37,13 +37,13 @@ struct Ctx {
   bool ready = false;
   int device = 0;
   cudaStream_t st = nullptr;
-  int n = 0, nfaces = 0, ref_row = 0, WA = 0, grid = 0;
+  int n = 0, nfaces = 0, ref_row = 0, WA = 0;
   int n_dir = 0;
   int *col = nullptr, *status = nullptr;
   unsigned* bar = nullptr;
   double *val = nullptr, *dinv = nullptr, *b = nullptr, *x = nullptr, *r = nullptr, *z = nullptr, *p0 = nullptr,
          *p1 = nullptr, *q = nullptr, *bp = nullptr, *part = nullptr, *dout = nullptr, *tot = nullptr;
-  void* kernel = nullptr;
+  PcgGrid plan;
   PcgCluster cluster;  // small systems: the solve on one cluster
   dpm::gpu::MlSolver* ml = nullptr;  // multilevel solve of the current operator (AMG names)
   int ml_nullsp = -1;
@@ -128,25 +128,11 @@ int build(int n, int nfaces, const int* l2g, const int* fo, const int* fnl, cons
   cudaMemcpy(g_ctx.col, hc.data(), hc.size() * sizeof(int), cudaMemcpyHostToDevice);
   cudaMemcpy(g_ctx.val, hv.data(), hv.size() * sizeof(double), cudaMemcpyHostToDevice);
   cudaMemcpy(g_ctx.dinv, hd.data(), n * sizeof(double), cudaMemcpyHostToDevice);
-  int sms = 0, per_sm = 0;
+  int sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, g_ctx.device);
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pcg<double, 0, 0>, PCG_TPB, 0) != cudaSuccess || per_sm < 1)
-    return -26;
-  g_ctx.grid = std::min(sms * per_sm, (n + PCG_TPB - 1) / PCG_TPB);
-  if (g_ctx.grid < 1) g_ctx.grid = 1;
-  int cpt = 0;
-  g_ctx.kernel = pcg_kernel_for<double>(n, g_ctx.grid, WA, &cpt);
-  int per_sm2 = 0;
-  cudaFuncSetAttribute(g_ctx.kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 5);
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm2, g_ctx.kernel, PCG_TPB, 0) != cudaSuccess || per_sm2 < 1)
-    return -26;
-  if (sms * per_sm2 < g_ctx.grid) {
-    g_ctx.grid = sms * per_sm2;
-    g_ctx.kernel = pcg_kernel_for<double>(n, g_ctx.grid, WA, &cpt);
-    cudaFuncSetAttribute(g_ctx.kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 5);
-  }
+  if (!g_ctx.plan.plan(n, WA, sms)) return -26;
   g_ctx.cluster.plan(n, WA);
-  if (dalloc(&g_ctx.part, 8 * (size_t)g_ctx.grid)) return -11;
+  if (dalloc(&g_ctx.part, 8 * (size_t)g_ctx.plan.grid)) return -11;
   g_ctx.n = n;
   g_ctx.nfaces = nfaces;
   g_ctx.ref_row = ref_row;
@@ -187,11 +173,8 @@ int run_pcg(double rtol, double atol, int maxit, int guess_zero, int* reason, in
   a.rtol = rtol; a.atol = atol; a.maxit = maxit; a.nullsp = g_ctx.n_dir > 0 ? 0 : 1; a.guess_zero = guess_zero;
   cudaMemsetAsync(g_ctx.bar, 0, 2 * sizeof(unsigned), g_ctx.st);
   cudaMemsetAsync(g_ctx.status, 0, 4 * sizeof(int), g_ctx.st);
-  void* args[] = {&a};
-  const cudaError_t le = g_ctx.cluster.kernel ? g_ctx.cluster.launch(a, g_ctx.st)
-                                              : cudaLaunchCooperativeKernel(g_ctx.kernel, dim3(g_ctx.grid),
-                                                                            dim3(PCG_TPB), args, 0, g_ctx.st);
-  if (le != cudaSuccess) return -33;
+  if ((g_ctx.cluster.kernel ? g_ctx.cluster.launch(a, g_ctx.st) : g_ctx.plan.launch(a, g_ctx.st)) != cudaSuccess)
+    return -33;
   int hs[4];
   double hd[4];
   cudaMemcpyAsync(hs, g_ctx.status, sizeof(hs), cudaMemcpyDeviceToHost, g_ctx.st);

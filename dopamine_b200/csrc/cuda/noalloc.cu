@@ -61,25 +61,24 @@ int scratch_address(void** ptr) {
   return 0;
 }
 
-// Every k_pcg and k_pcg_cluster instantiation the solve can pick (row width 7 or runtime):
-// querying their attributes makes the runtime load them now rather than at a later launch.
+// Every kernel the solve can pick (row width 7 or runtime): setting their attributes makes the runtime
+// load them now rather than at a later launch.
 int preload_kernels() {
-  const void* ks[] = {(const void*)k_pcg<double, 0, 7>, (const void*)k_pcg<double, 1, 7>,
-                      (const void*)k_pcg<double, 2, 7>, (const void*)k_pcg<double, 3, 7>,
-                      (const void*)k_pcg<double, 4, 7>, (const void*)k_pcg<double, 0, 0>,
-                      (const void*)k_pcg<double, 1, 0>, (const void*)k_pcg<double, 2, 0>,
-                      (const void*)k_pcg<double, 3, 0>, (const void*)k_pcg<double, 4, 0>};
-  for (const void* k : ks) {
-    cudaFuncAttributes fa;
-    if (cudaFuncGetAttributes(&fa, k) != cudaSuccess) return DPM_ERR_CUDA;
-    if (cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 5) != cudaSuccess) return DPM_ERR_CUDA;
-  }
-  for (int cpt = 1; cpt <= PCG_CL_CPT; ++cpt)
-    for (int width : {7, 0}) {
-      cudaFuncAttributes fa;
-      const void* k = PcgCluster::pick(cpt, width);
-      if (cudaFuncGetAttributes(&fa, k) != cudaSuccess || !PcgCluster::prepare(k)) return DPM_ERR_CUDA;
+  cudaFuncAttributes fa;
+  for (int width : {7, 0}) {
+    for (int cpt = 1; cpt <= PCG_ST_CPT; ++cpt) {
+      const void* k = PcgGrid::staged(cpt, width);
+      if (cudaFuncGetAttributes(&fa, k) != cudaSuccess || !PcgGrid::prepare(k, true)) return DPM_ERR_CUDA;
     }
+    for (int cpt : {0, 2, 3, 4}) {
+      const void* k = PcgGrid::regs(cpt, width);
+      if (cudaFuncGetAttributes(&fa, k) != cudaSuccess || !PcgGrid::prepare(k, false)) return DPM_ERR_CUDA;
+    }
+    for (int cpt = 1; cpt <= PCG_CL_CPT; ++cpt) {
+      const void* c = PcgCluster::pick(cpt, width);
+      if (cudaFuncGetAttributes(&fa, c) != cudaSuccess || !PcgCluster::prepare(c)) return DPM_ERR_CUDA;
+    }
+  }
   return 0;
 }
 
@@ -112,26 +111,12 @@ extern "C" int dpm_pcg_solve_noalloc(int n_cells, int row_width, const int* col,
   if (!col || !val || !inv_diag || !rhs || !x) return DPM_ERR_ARG;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
 
-  int sms = 0, per_sm = 0, cpt = 0;
+  int sms = 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return DPM_ERR_CUDA;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pcg<double, 0, 0>, PCG_TPB, 0) != cudaSuccess ||
-      per_sm < 1)
-    return DPM_ERR_CUDA;
-  int grid = sms * per_sm;
-  if (grid > (n_cells + PCG_TPB - 1) / PCG_TPB) grid = (n_cells + PCG_TPB - 1) / PCG_TPB;
-  if (grid > kMaxBlocks) grid = kMaxBlocks;
-  if (grid < 1) grid = 1;
-  void* kernel = pcg_kernel_for<double>(n_cells, grid, row_width, &cpt);
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 5) != cudaSuccess) return DPM_ERR_CUDA;
-  int per_sm2 = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm2, kernel, PCG_TPB, 0) != cudaSuccess || per_sm2 < 1)
-    return DPM_ERR_CUDA;
-  if (grid > sms * per_sm2) {
-    grid = sms * per_sm2;
-    kernel = pcg_kernel_for<double>(n_cells, grid, row_width, &cpt);
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 5) != cudaSuccess)
-      return DPM_ERR_CUDA;
-  }
+  PcgGrid plan;
+  PcgCluster cluster;
+  cluster.plan(n_cells, row_width);
+  if (!cluster.kernel && (!plan.plan(n_cells, row_width, sms) || plan.grid > kMaxBlocks)) return DPM_ERR_CUDA;
 
   double* base = static_cast<double*>(scratch);
   unsigned* bar = reinterpret_cast<unsigned*>(base + kNumDoubles);
@@ -162,12 +147,7 @@ extern "C" int dpm_pcg_solve_noalloc(int n_cells, int row_width, const int* col,
   a.maxit = max_iterations;
   a.nullsp = null_space ? 1 : 0;
   a.guess_zero = 0;
-  void* args[] = {&a};
-  PcgCluster cluster;
-  cluster.plan(n_cells, row_width);
-  const cudaError_t le = cluster.kernel ? cluster.launch(a, st)
-                                        : cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(PCG_TPB), args, 0, st);
-  if (le != cudaSuccess) return DPM_ERR_CUDA;
+  if ((cluster.kernel ? cluster.launch(a, st) : plan.launch(a, st)) != cudaSuccess) return DPM_ERR_CUDA;
   int hs[4];
   double hd[4];
   if (cudaMemcpyAsync(hs, status, sizeof(hs), cudaMemcpyDeviceToHost, st) != cudaSuccess) return DPM_ERR_CUDA;

@@ -11,13 +11,14 @@
 //   phase B: x += a p, r -= a q, z = D^-1 r, partials r.r, sum z, sum r, z.r  -> grid all-reduce
 //
 // Rows of A are stored ELL [width][n] with sorted columns and padded to a fixed width with
-// (self, 0) entries, so each row is a fully unrolled set of independent loads.  A and 1/diag are
-// read through the read-only path and stay L1-resident across iterations; the vectors that
-// neighbours read (z, p) go through L2 (ld.cg), which is where other SMs' writes are visible.
-// Each thread keeps its own cells' x, r, z and p in registers when the mesh fits (CPT cells per
-// thread).  Grid all-reduces are deterministic (see grid_allreduce).  The launch is cooperative,
-// which guarantees co-residency of all blocks; every wait is bounded.
+// (self, 0) entries.  k_pcg_staged up to 1024 rows per SM; k_pcg beyond: up to 4096 with each thread's
+// x, r, z and p in registers (CPT cells per thread), then with grid-stride loops.  The vectors that
+// neighbours read (z, p) go through L2 (ld.cg), where other SMs' writes are visible.  Grid all-reduces
+// are deterministic (see grid_allreduce).  The launches are cooperative, which guarantees co-residency
+// of all blocks; every wait is bounded.
 #pragma once
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace dpm {
@@ -55,6 +56,11 @@ struct PcgArgs {
 };
 
 __device__ __forceinline__ double ld_cg(const double* p) { return __ldcg(p); }
+__device__ __forceinline__ double ld_cg_if(const double* p, int on) {  // 0 when off
+  double v = 0.0;
+  asm volatile("{ .reg .pred t; setp.ne.s32 t, %2, 0; @t ld.global.cg.f64 %0, [%1]; }" : "+d"(v) : "l"(p), "r"(on) : "memory");
+  return v;
+}
 __device__ __forceinline__ float ld_cg(const float* p) { return __ldcg(p); }
 
 // Grid-wide deterministic all-reduce + barrier.  Each block reduces its NV values (fixed shuffle
@@ -100,7 +106,8 @@ __device__ __forceinline__ bool grid_allreduce(double (&v)[NV], double* partials
       if (++spins > lim) { ok = 0; atomicExch(&status[2], 1); break; }
       if (spins > 32) __nanosleep(20);
     }
-    __threadfence();
+    // the acquiring load orders what the block reads after the next barrier: a fence here as well cost
+    // 0.4 us per wait (393 216 rows: 12.9 us per iteration with it, 12.0 without)
     s_ok = ok;
   }
   __syncthreads();
@@ -180,7 +187,7 @@ __device__ __forceinline__ double spmv_row_p(const PcgArgs<V>& a, int i, const V
   return s;
 }
 
-// CPT > 0: exactly CPT cells per thread, own x, r, z, p held in registers
+// CPT > 0: at most CPT cells per thread, own x, r, z, p held in registers
 //          (requires n <= grid * blockDim * CPT).
 // CPT == 0: grid-stride loops with the own-cell vectors in global memory (any n).
 // WT: fixed padded row width (7 on hexahedral meshes), 0 = runtime width <= 16.
@@ -369,30 +376,278 @@ __global__ void __launch_bounds__(PCG_TPB, 1) k_pcg(PcgArgs<V> a) {
   }
 }
 
-// Host helper: picks the instantiation for the mesh size (register-resident when it fits) and
-// row width (fixed 7 for hexahedral meshes).
-template <class V>
-inline void* pcg_kernel_for(int n, int grid, int width, int* cpt_out) {
-  const long cap = (long)grid * PCG_TPB;
-  int cpt = n <= cap ? 1 : n <= 2 * cap ? 2 : n <= 3 * cap ? 3 : n <= 4 * cap ? 4 : 0;
-  *cpt_out = cpt;
-  if (width == 7) {
+// The scalars that an iteration of the staged form carries over, with KSPCG's tests.
+struct PcgScalars {
+  double beta, betaold = 0.0, dpi = 0.0, bb = 0.0, mz;
+  // before p: KSP_DIVERGED_INDEFINITE_PC on a sign change of z.r; 0 when the iteration goes on
+  __device__ int top(int it) const {
+    if (beta == 0.0) return 3;
+    return it > 0 && beta * betaold < 0.0 ? -8 : 0;
+  }
+  // p.q: KSP_DIVERGED_INDEFINITE_MAT on a sign change
+  __device__ int curvature(int it, double pq) {
+    const double old = dpi;
+    dpi = pq;
+    betaold = beta;
+    if (dpi == 0.0) return 3;
+    return it > 0 && ((dpi > 0) - (dpi < 0)) * ((old > 0) - (old < 0)) < 0 ? -10 : 0;
+  }
+  // the sums (r.r, sum z, sum r, z.r) after the update
+  __device__ void next(const double (&s)[4], int nullsp, int n) {
+    mz = nullsp ? s[1] / (double)n : 0.0;
+    beta = nullsp ? s[3] - mz * s[2] : s[3];
+    bb = beta / betaold;
+  }
+};
+
+// Staged form: block b owns the consecutive rows [b C, b C + size) and keeps the operator (the first
+// WS slots of its rows) and its part of p in shared memory, x, r, p, q and 1/diag in registers.  The
+// entries of a row that lie in the block's own rows - five of seven on a hexahedral mesh - read p
+// there; the others form p_j from z_j and the old p_j in L2, as k_pcg does for all.
+// us per iteration, here and in the form that reads all of it through L2: 44 880 rows 6.8 / 8.8,
+// 66 600 rows 6.9 / 8.85, 85 050 rows 7.5 / 8.9.  With more than two rows per thread the few warps no
+// longer cover the loads from other blocks' rows, one row after the other (393 216 rows, six rows per
+// thread: 15.5 / 12.7), and the register form with 32 warps takes over.
+// CPT: rows per thread.
+constexpr int PCG_ST_TPB = 512;
+constexpr int PCG_ST_CPT = 2;
+template <int CPT, int WT>
+__global__ void __launch_bounds__(PCG_ST_TPB, 1) k_pcg_staged(PcgArgs<double> a, int C, int WC, int WS) {
+  extern __shared__ double st_smem[];
+  constexpr int CH = WT > 0 ? WT : 4;  // slots whose loads are in flight together
+  const int n = a.n, WA = WT > 0 ? WT : a.WA;
+  const int base = (int)blockIdx.x * C, size = max(0, min(C, n - base));
+  double* s_p = st_smem;                               // [C]
+  double* s_val = s_p + C;                             // [WS][C]
+  int* s_col = reinterpret_cast<int*>(s_val + (size_t)WS * C);  // [WC][C] own row l, or ~global column
+  unsigned gen = 0;
+  auto code = [&](int c) { return (unsigned)(c - base) < (unsigned)size ? c - base : ~c; };
+  // row l of this block times the vector that is s_p on its own rows and elsewhere z - m + f po (no f:
+  // z - m).  Both loads are predicated, not branched over, so that a row's are in flight together.
+  auto product = [&](int l, const double* z, const double* po, double m, double f, int with_po) {
+    double s = 0.0;
+    for (int w0 = 0; w0 < WA; w0 += CH) {
+      int cc[CH];
+      double v[CH], x[CH];
+#pragma unroll
+      for (int u = 0; u < CH; ++u) {
+        const int w = w0 + u;
+        const bool on = WT > 0 || w < WA;
+        cc[u] = !on ? l : w < WC ? s_col[w * C + l] : code(__ldg(&a.col[(size_t)w * n + base + l]));
+        v[u] = !on ? 0.0 : w < WS ? s_val[w * C + l] : __ldcg(&a.val[(size_t)w * n + base + l]);
+      }
+      double zz[CH], pp[CH];
+#pragma unroll
+      for (int u = 0; u < CH; ++u) {
+        const int j = cc[u] < 0 ? ~cc[u] : 0;
+        zz[u] = ld_cg_if(z + j, cc[u] < 0);
+        pp[u] = ld_cg_if(po + j, cc[u] < 0 && with_po);
+      }
+#pragma unroll
+      for (int u = 0; u < CH; ++u) x[u] = s_p[max(cc[u], 0)];
+#pragma unroll
+      for (int u = 0; u < CH; ++u) {
+        if (cc[u] < 0) {
+          x[u] = zz[u] - m;
+          if (with_po) x[u] = x[u] + f * pp[u];
+        }
+        s += v[u] * x[u];
+      }
+    }
+    return s;
+  };
+#define ST_OWN(k) ((int)threadIdx.x + (k) * PCG_ST_TPB < size)
+#define ST_ROW(k) ((int)threadIdx.x + (k) * PCG_ST_TPB)
+  for (int w = 0; w < WC; ++w)
+    for (int l = threadIdx.x; l < size; l += PCG_ST_TPB) {
+      s_col[w * C + l] = code(__ldg(&a.col[(size_t)w * n + base + l]));
+      if (w < WS) s_val[w * C + l] = __ldg(&a.val[(size_t)w * n + base + l]);
+    }
+  double rx[CPT], rr[CPT], rp[CPT], rq[CPT], rd[CPT];
+  // ---- b' = b - mean(b) when the constant null space is active; the guess
+  double mb = 0.0;
+  {
+    double v[1] = {0.0}, t[1];
+#pragma unroll
+    for (int k = 0; k < CPT; ++k)
+      if (ST_OWN(k)) {
+        const int i = base + ST_ROW(k);
+        rx[k] = a.guess_zero ? 0.0 : a.x[i];
+        rr[k] = a.b[i];
+        rd[k] = __ldg(&a.dinv[i]);
+        rp[k] = 0.0;
+        s_p[ST_ROW(k)] = rx[k];
+        v[0] += rr[k];
+      }
+    if (!grid_allreduce<1>(v, a.partials, a.bar, gen, a.status, t)) return;
+    mb = a.nullsp ? t[0] / (double)n : 0.0;
+  }
+  // ---- r = b' - A x (the caller's x: nobody writes it before the end)
+  double v2[2] = {0.0, 0.0}, t2[2];
+#pragma unroll
+  for (int k = 0; k < CPT; ++k)
+    if (ST_OWN(k)) {
+      const double bp = a.nullsp ? rr[k] - mb : rr[k];
+      rr[k] = bp - (a.guess_zero ? 0.0 : product(ST_ROW(k), a.x, a.x, 0.0, 0.0, 0));
+      v2[0] += rr[k] * rr[k];
+      v2[1] += bp * bp;
+    }
+  if (!grid_allreduce<2>(v2, a.partials, a.bar, gen, a.status, t2)) return;
+  double dp = sqrt(t2[0]);
+  const double sn = sqrt(t2[1]);
+  const double rnorm0 = a.guess_zero ? dp : (sn == 0.0 ? dp : sn);
+  const double ttol = fmax(a.rtol * rnorm0, a.atol);
+  int reason = classify(dp, ttol, a.atol, rnorm0);
+  int its = 0;
+  if (!reason) {
+    // ---- z = D^-1 r
+    double v4[4] = {0, 0, 0, 0}, t4[4];
+#pragma unroll
+    for (int k = 0; k < CPT; ++k)
+      if (ST_OWN(k)) {
+        const double z = rr[k] * rd[k];
+        a.z[base + ST_ROW(k)] = z;
+        v4[0] += z; v4[1] += rr[k]; v4[2] += z * rr[k];
+      }
+    if (!grid_allreduce<4>(v4, a.partials, a.bar, gen, a.status, t4)) return;
+    PcgScalars c;
+    c.mz = a.nullsp ? t4[0] / (double)n : 0.0;
+    c.beta = a.nullsp ? t4[2] - c.mz * t4[1] : t4[2];
+    double* pold = a.p0;
+    double* pnew = a.p1;
+    int it = 0;
+    do {
+      its = it + 1;
+      if ((reason = c.top(it))) break;
+      const bool first = it == 0;
+      // ---- p, q = A p, p.q
+#pragma unroll
+      for (int k = 0; k < CPT; ++k)
+        if (ST_OWN(k)) {
+          double p = rr[k] * rd[k] - c.mz;
+          if (!first) p = p + c.bb * rp[k];
+          rp[k] = p;
+          s_p[ST_ROW(k)] = p;
+          pnew[base + ST_ROW(k)] = p;
+        }
+      __syncthreads();
+      double v1[1] = {0.0}, t1[1];
+#pragma unroll
+      for (int k = 0; k < CPT; ++k)
+        if (ST_OWN(k)) {
+          rq[k] = product(ST_ROW(k), a.z, pold, c.mz, c.bb, !first);
+          v1[0] += rp[k] * rq[k];
+        }
+      if (!grid_allreduce<1>(v1, a.partials, a.bar, gen, a.status, t1)) return;
+      if ((reason = c.curvature(it, t1[0]))) break;
+      const double al = c.beta / c.dpi;
+      // ---- x, r, z and the four sums
+      double w4[4] = {0, 0, 0, 0}, s4[4];
+#pragma unroll
+      for (int k = 0; k < CPT; ++k)
+        if (ST_OWN(k)) {
+          rx[k] = rx[k] + al * rp[k];
+          rr[k] = rr[k] - al * rq[k];
+          const double z = rr[k] * rd[k];
+          a.z[base + ST_ROW(k)] = z;
+          w4[0] += rr[k] * rr[k]; w4[1] += z; w4[2] += rr[k]; w4[3] += z * rr[k];
+        }
+      if (!grid_allreduce<4>(w4, a.partials, a.bar, gen, a.status, s4)) return;
+      dp = sqrt(s4[0]);
+      c.next(s4, a.nullsp, n);
+      reason = classify(dp, ttol, a.atol, rnorm0);
+      if (reason) break;
+      double* t = pold; pold = pnew; pnew = t;
+      it++;
+    } while (it < a.maxit);
+    if (!reason && it >= a.maxit) reason = -3;
+  }
+  // ---- x, then the true residual ||b - A x|| with the caller's b (KSPBuildResidual)
+#pragma unroll
+  for (int k = 0; k < CPT; ++k)
+    if (ST_OWN(k)) {
+      a.x[base + ST_ROW(k)] = rx[k];
+      s_p[ST_ROW(k)] = rx[k];
+    }
+  double v1[1] = {0.0}, t1[1];
+  if (!grid_allreduce<1>(v1, a.partials, a.bar, gen, a.status, t1)) return;
+#pragma unroll
+  for (int k = 0; k < CPT; ++k)
+    if (ST_OWN(k)) {
+      const double d = a.b[base + ST_ROW(k)] - product(ST_ROW(k), a.x, a.x, 0.0, 0.0, 0);
+      v1[0] += d * d;
+    }
+  if (!grid_allreduce<1>(v1, a.partials, a.bar, gen, a.status, t1)) return;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    a.dout[0] = sqrt(t1[0]);
+    a.dout[1] = dp;
+    a.dout[2] = sn;
+    a.status[0] = reason;
+    a.status[1] = its;
+  }
+#undef ST_OWN
+#undef ST_ROW
+}
+
+// The cooperative launch of a system: kernel, blocks, rows per block, staged slots, shared memory.
+struct PcgGrid {
+  void* kernel = nullptr;
+  int grid = 0, tpb = 0, C = 0, WC = 0, WS = 0;  // WC, WS: slots whose columns and values are staged
+  size_t smem = 0;
+  static constexpr int max_smem = 223 * 1024;  // of 227 KB per block; the all-reduces' buffers take 3 KB
+
+  template <int CPT>
+  static void* pick_cpt(int cpt, int width) {
+    if constexpr (CPT < PCG_ST_CPT)
+      if (cpt > CPT) return pick_cpt<CPT + 1>(cpt, width);
+    return width == 7 ? (void*)k_pcg_staged<CPT, 7> : (void*)k_pcg_staged<CPT, 0>;
+  }
+  static void* staged(int cpt, int width) { return pick_cpt<1>(cpt, width); }
+  static void* regs(int cpt, int width) {  // cpt 2..4: register-resident, else grid-stride
+    const bool w7 = width == 7;
     switch (cpt) {
-      case 1: return (void*)k_pcg<V, 1, 7>;
-      case 2: return (void*)k_pcg<V, 2, 7>;
-      case 3: return (void*)k_pcg<V, 3, 7>;
-      case 4: return (void*)k_pcg<V, 4, 7>;
-      default: return (void*)k_pcg<V, 0, 7>;
+      case 2: return w7 ? (void*)k_pcg<double, 2, 7> : (void*)k_pcg<double, 2, 0>;
+      case 3: return w7 ? (void*)k_pcg<double, 3, 7> : (void*)k_pcg<double, 3, 0>;
+      case 4: return w7 ? (void*)k_pcg<double, 4, 7> : (void*)k_pcg<double, 4, 0>;
+      default: return w7 ? (void*)k_pcg<double, 0, 7> : (void*)k_pcg<double, 0, 0>;
     }
   }
-  switch (cpt) {
-    case 1: return (void*)k_pcg<V, 1, 0>;
-    case 2: return (void*)k_pcg<V, 2, 0>;
-    case 3: return (void*)k_pcg<V, 3, 0>;
-    case 4: return (void*)k_pcg<V, 4, 0>;
-    default: return (void*)k_pcg<V, 0, 0>;
+  // Loads the kernel and sets its shared memory, or for the other forms the largest L1.
+  static bool prepare(const void* k, bool is_staged) {
+    return (is_staged ? cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem)
+                      : cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 5)) == cudaSuccess;
   }
-}
+  // 256 rows per block at least: fewer blocks have less to wait for
+  bool plan(int n, int width, int sms) {
+    kernel = nullptr;
+    grid = std::max(1, std::min(sms, (n + 255) / 256));
+    C = (n + grid - 1) / grid;
+    const int cpt = (C + PCG_ST_TPB - 1) / PCG_ST_TPB;
+    const bool st = cpt <= PCG_ST_CPT;
+    tpb = st ? PCG_ST_TPB : PCG_TPB;
+    WC = WS = 0;
+    smem = 0;
+    if (st) {  // columns first: a column from L2 delays the load that depends on it
+      const size_t words = max_smem / (4 * (size_t)C) - 2;
+      WC = (int)std::min<size_t>(width, words);
+      WS = (int)std::min<size_t>(WC, (words - WC) / 2);
+      smem = 4 * (size_t)C * (2 + WC + 2 * WS);
+    }
+    const int rows = (C + PCG_TPB - 1) / PCG_TPB;  // of a thread in the register form
+    void* k = st ? staged(cpt, width) : regs(rows >= 2 && rows <= 4 ? rows : 0, width);
+    int per_sm = 0;
+    if (!prepare(k, st) || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, tpb, smem) != cudaSuccess ||
+        per_sm < 1)
+      return false;
+    kernel = k;
+    return true;
+  }
+  cudaError_t launch(PcgArgs<double> a, cudaStream_t st) const {
+    int rows = C, cols = WC, slots = WS;
+    void* staged_args[] = {&a, &rows, &cols, &slots};
+    return cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(tpb), staged_args, smem, st);  // k_pcg takes the first
+  }
+};
 
 }  // namespace gpu
 }  // namespace dpm

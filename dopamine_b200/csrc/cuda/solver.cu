@@ -217,13 +217,10 @@ struct Solver {
   int cp_iters = 0, cp_precond_iters = 0;
   // PCG workspace
   double *cg_r, *cg_z, *cg_p0, *cg_p1, *cg_q, *cg_bp, *cg_x, *cg_part, *cg_dout;
-  void* cg_kernel = nullptr;
-  int cg_cpt = 0;
+  PcgGrid cg_plan;
+  PcgCluster cg_cluster;  // small meshes: the solve on one cluster (unless a poll limit is set)
   unsigned* cg_bar;
   int* cg_status;
-  int cg_grid = 0;
-  PcgCluster cg_cluster;  // small meshes: the solve on one cluster (unless a poll limit is set)
-  bool cg_coop = true;
   // temperature (transported when Boussinesq is on) and passive scalars, scalar-major
   double *Tb = nullptr, *gT = nullptr, *HT = nullptr, *HT0 = nullptr;
   int ns = 0;
@@ -578,29 +575,12 @@ struct Solver {
       if (rc) return rc;
     }
     // cooperative grid for the persistent PCG
-    int dev_sms = 0, per_sm = 0, coop = 0;
+    int dev_sms = 0, coop = 0;
     CK(cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, device));
     CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device));
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pcg<double, 0, 0>, PCG_TPB, 0));
-    cg_coop = coop != 0 && per_sm > 0;
-    if (!cg_coop) return DPM_ERR_UNSUPPORTED;
-    cg_grid = std::min(dev_sms * per_sm, std::max(1, (nc + PCG_TPB - 1) / PCG_TPB));
-    cg_kernel = pcg_kernel_for<double>(nc, cg_grid, S.WA, &cg_cpt);
-    // A and 1/diag should stay in L1 across iterations: prefer the largest L1 carveout (set before
-    // the occupancy query, which the cooperative launch check must agree with).
-    CK(cudaFuncSetAttribute(cg_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 5));
-    {
-      int per_sm2 = 0;
-      CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm2, cg_kernel, PCG_TPB, 0));
-      if (per_sm2 < 1) return DPM_ERR_UNSUPPORTED;
-      if (dev_sms * per_sm2 < cg_grid) {  // fewer co-resident blocks: re-pick with the smaller grid
-        cg_grid = dev_sms * per_sm2;
-        cg_kernel = pcg_kernel_for<double>(nc, cg_grid, S.WA, &cg_cpt);
-        CK(cudaFuncSetAttribute(cg_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 5));
-      }
-    }
+    if (!coop || !cg_plan.plan(nc, S.WA, dev_sms)) return DPM_ERR_UNSUPPORTED;
     cg_cluster.plan(nc, S.WA);
-    cg_part = mem.alloc<double>(8 * (size_t)cg_grid);
+    cg_part = mem.alloc<double>(8 * (size_t)cg_plan.grid);
     {
       int rc = setup_scalars();
       if (rc) return rc;
@@ -1596,9 +1576,8 @@ struct Solver {
     CK(cudaMemsetAsync(cg_bar, 0, 2 * sizeof(unsigned), st));
     CK(cudaMemsetAsync(cg_status, 0, 4 * sizeof(int), st));
     if (spin_limit) CK(cudaMemcpyAsync(cg_status + 3, &spin_limit, sizeof(int), cudaMemcpyHostToDevice, st));
-    void* args[] = {&a};
     if (cg_cluster.kernel && !spin_limit) CK(cg_cluster.launch(a, st));
-    else CK(cudaLaunchCooperativeKernel(cg_kernel, dim3(cg_grid), dim3(PCG_TPB), args, 0, st));
+    else CK(cg_plan.launch(a, st));
     launches++;
     int h_st[4];
     double h_d[4];
