@@ -278,7 +278,7 @@ def run_gpu(args, rank, world):
     torch.cuda.set_device(dev)
     case = make_case(args.config)
     if args.psolver == "auto":
-        case.params["p_solver"] = 3  # DPM_PSOLVER_AUTO: two-level when the mesh fits it, else multilevel
+        case.params["p_solver"] = 3  # DPM_PSOLVER_AUTO: two-level up to 131 072 cells, else multilevel
     if args.psolver == "ml":
         case.params["p_solver"] = 2  # DPM_PSOLVER_MULTILEVEL_FCG
     if args.psolver == "fcg":
@@ -422,7 +422,7 @@ def main():
     ap.add_argument("--fcg-phases", action="store_true",
                     help="after the timed region, record the two-level kernel's phase times for 2 steps")
     ap.add_argument("--psolver", default="auto", choices=["auto", "pcg", "fcg", "ml"],
-                    help="auto: fcg when the mesh fits the two-level kernel, else ml; pcg: plain FP64 "
+                    help="auto: fcg up to 131 072 cells, else ml; pcg: plain FP64 "
                          "Jacobi-PCG; fcg: flexible CG, two-level part-local preconditioner; "
                          "ml: flexible CG, aggregation-multigrid V-cycle")
     args = ap.parse_args()

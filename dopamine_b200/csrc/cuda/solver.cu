@@ -78,6 +78,8 @@ struct DMem {
   }
 };
 
+constexpr int AUTO_TWOLEVEL_CELLS = 1 << 17;  // DPM_PSOLVER_AUTO: two-level up to here
+
 inline int nblk(int64_t n) { return (int)((n + TPB - 1) / TPB); }
 
 // ---- deterministic reductions: per-block partials, then one block sums them in order --------
@@ -596,8 +598,12 @@ struct Solver {
       int rc = setup_ml(dev_sms);
       if (rc) return rc;
     } else if (P.p_solver == DPM_PSOLVER_AUTO) {
-      // the two-level kernel keeps a part of <= 4096 cells per block, one block per SM
-      int rc = (nc + dev_sms - 1) / dev_sms <= 4096 ? setup_fcg(dev_sms) : DPM_ERR_UNSUPPORTED;
+      // The two-level kernel keeps a part of <= 4096 cells per block, one block per SM; its iterations
+      // cost 14-27 us and their number grows with the mesh.  Poisson ms per step, two-level and
+      // multilevel: 108 000 cells 3.5 / 3.7 and 5.7 / 5.9, 148 640 cells 6.9 / 6.5, 175 616 cells
+      // 4.5 / 3.5, 393 216 cells 9.6 / 6.6.
+      int rc = nc <= AUTO_TWOLEVEL_CELLS && (nc + dev_sms - 1) / dev_sms <= 4096 ? setup_fcg(dev_sms)
+                                                                                 : DPM_ERR_UNSUPPORTED;
       if (rc == DPM_ERR_UNSUPPORTED) rc = setup_ml(dev_sms);
       if (rc) return rc;
     } else if (P.p_solver != DPM_PSOLVER_JACOBI_PCG) {
