@@ -15,7 +15,9 @@
 // 50 400 rows 10.6 / 8.8).
 //
 // Its waits need no poll limit: the blocks of a cluster are scheduled together, and every thread
-// reaches every barrier.
+// reaches every barrier.  Scheduled together does not mean started: a block's shared memory may be
+// accessed only once that block runs, so each block arrives at a cluster barrier on entry and waits
+// there after staging its operator, before the first store to another block.
 #pragma once
 #include <algorithm>
 
@@ -47,9 +49,11 @@ __device__ __forceinline__ double cl_ld(unsigned addr) {
 __device__ __forceinline__ void cl_st(unsigned addr, double v) {
   asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(addr), "d"(v) : "memory");
 }
+__device__ __forceinline__ void cl_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cl_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cl_barrier() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  cl_arrive();
+  cl_wait();
 }
 
 // Sums over a warp of four values at once: two exchange steps leave each lane one value's partial
@@ -105,6 +109,7 @@ __device__ __forceinline__ void cl_allreduce(const double (&v)[4], double (&res)
 template <int CPT, int WT>
 __global__ void __launch_bounds__(PCG_CL_TPB, 1) k_pcg_cluster(PcgArgs<double> a, int C, int WS) {
   extern __shared__ double cl_smem[];
+  cl_arrive();                            // this block runs; cl_wait below: all blocks do
   constexpr int CH = WT > 0 ? WT : 4;     // slots whose loads are in flight together
   const int n = a.n, WA = WT > 0 ? WT : a.WA;
   const unsigned rank = cl_rank(), nblk = gridDim.x;
@@ -157,6 +162,7 @@ __global__ void __launch_bounds__(PCG_CL_TPB, 1) k_pcg_cluster(PcgArgs<double> a
       s_adr[w * C + l] = address(__ldg(&a.col[(size_t)w * n + base + l]));
       s_val[w * C + l] = __ldg(&a.val[(size_t)w * n + base + l]);
     }
+  cl_wait();
   double rx[CPT], rr[CPT], rp[CPT], rq[CPT], rd[CPT];
   // ---- b' = b - mean(b) when the constant null space is active; x published
   double mb = 0.0;
