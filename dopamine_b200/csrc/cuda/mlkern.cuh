@@ -47,10 +47,30 @@ struct MlkState {
 
 // The kernels of an iteration are launched with programmatic stream serialization: each lets the
 // next one's blocks come in as its own drain, and waits here for the one before to have completed
-// (its stores visible) before it touches memory.
+// (its stores visible) before it touches memory.  A kernel is thus resident while the arrays that it
+// reads are still being written: those are read by mlk_ld, __ldcg or plain loads, which stay behind the
+// wait, never by __ldg (the non-coherent load wants data that nobody writes while the kernel lives, and
+// may be moved up) nor through __restrict__ pointers (which the clobbers above do not cover).  __ldg
+// is for what the set-up wrote: operators, transfers, diagonals, the inverse, omega.
 __device__ __forceinline__ void mlk_enter() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+// A cached load of such a value; not reordered with mlk_enter.
+__device__ __forceinline__ float mlk_ld(const float* p) {
+  float v;
+  asm volatile("ld.global.ca.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float mlk_ld_if(const float* p, bool on) {  // 0 when off
+  float v = 0.0f;
+  asm volatile("{ .reg .pred t; setp.ne.s32 t, %2, 0; @t ld.global.ca.f32 %0, [%1]; }" : "+f"(v) : "l"(p), "r"((int)on));
+  return v;
+}
+__device__ __forceinline__ float4 mlk_ld(const float4* p) {
+  float4 v;
+  asm volatile("ld.global.ca.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+  return v;
 }
 
 // Block sum of NV values per thread into part[block][NV] (fixed shuffle tree, then warps in order).
@@ -150,10 +170,10 @@ static __global__ void __launch_bounds__(256) k_mlk_first(MlkLevel L, const MlkS
 
 // Row sum of val * v[index] for the row of this thread (SELL: thread = row; else 2^lg lanes per
 // row, every lane of the row returning the sum, added over the lanes by a fixed butterfly).  A
-// lane's loads are in flight together, eight or four at a time.  v is not written by the kernel,
-// so the gathers go through L1: neighbouring rows share most of their columns.
+// lane's loads are in flight together, eight or four at a time.  The gathers go through L1:
+// neighbouring rows share most of their columns.
 template <bool SELL>
-__device__ __forceinline__ float mlk_rowsum(const MlkRows& m, int t, int rows, const float* __restrict__ v) {
+__device__ __forceinline__ float mlk_rowsum(const MlkRows& m, int t, int rows, const float* v) {
   float s = 0.0f;
   if (SELL) {
     if (t >= rows) return s;
@@ -166,13 +186,13 @@ __device__ __forceinline__ float mlk_rowsum(const MlkRows& m, int t, int rows, c
 #pragma unroll
       for (int u = 0; u < 8; ++u) e[u] = __ldg(&q[32 * (k + u)]);
 #pragma unroll
-      for (int u = 0; u < 8; ++u) x[u] = __ldg(&v[e[u].x]);
+      for (int u = 0; u < 8; ++u) x[u] = mlk_ld(&v[e[u].x]);
 #pragma unroll
       for (int u = 0; u < 8; ++u) s = fmaf(__int_as_float(e[u].y), x[u], s);
     }
     for (; k < w; ++k) {
       const int2 e = __ldg(&q[32 * k]);
-      s = fmaf(__int_as_float(e.y), __ldg(&v[e.x]), s);
+      s = fmaf(__int_as_float(e.y), mlk_ld(&v[e.x]), s);
     }
     return s;
   }
@@ -185,7 +205,7 @@ __device__ __forceinline__ float mlk_rowsum(const MlkRows& m, int t, int rows, c
 #pragma unroll
     for (int u = 0; u < 4; ++u) q[u] = e + u * G < e1 ? __ldg(&m.ent[e + u * G]) : make_int2(-1, 0);
 #pragma unroll
-    for (int u = 0; u < 4; ++u) x[u] = q[u].x >= 0 ? __ldg(&v[q[u].x]) : 0.0f;
+    for (int u = 0; u < 4; ++u) x[u] = mlk_ld_if(v + max(q[u].x, 0), q[u].x >= 0);
 #pragma unroll
     for (int u = 0; u < 4; ++u) s = fmaf(__int_as_float(q[u].y), x[u], s);
   }
@@ -265,7 +285,7 @@ __device__ __forceinline__ float mlk_row0(const MlkLevel& L, int i, const float*
       v[u] = k0 + u < L.W ? ml_sval(&sv[e]) : 0.0f;
     }
 #pragma unroll
-    for (int u = 0; u < ML_CHUNK; ++u) xv[u] = __ldg(&x[c[u]]);
+    for (int u = 0; u < ML_CHUNK; ++u) xv[u] = mlk_ld(&x[c[u]]);
 #pragma unroll
     for (int u = 0; u < ML_CHUNK; ++u) s = fmaf(v[u], xv[u], s);
   }
@@ -273,33 +293,33 @@ __device__ __forceinline__ float mlk_row0(const MlkLevel& L, int i, const float*
 }
 template <class SV>
 static __global__ void __launch_bounds__(MLK_TPB) k_mlk_sweep(MlkLevel L, int step, int keep, float c1, float c2,
-                                                       const float* __restrict__ xi, float* __restrict__ xo,
-                                                       const float* __restrict__ om, float gam, const MlkState* S) {
+                                                       const float* xi, float* xo,
+                                                       const float* om, float gam, const MlkState* S) {
   mlk_enter();
   if (S->done) return;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= L.n) return;
   const float acc = mlk_row0<SV>(L, i, xi);
-  mlk_step(L, step, keep, c1, c2, i, acc, __ldg(&xi[i]), xo, om ? gam * __ldg(&om[i]) : 0.0f);
+  mlk_step(L, step, keep, c1, c2, i, acc, mlk_ld(&xi[i]), xo, om ? gam * __ldg(&om[i]) : 0.0f);
 }
 // Other levels, 30-110 entries per row: a row per thread in 32-row slices while the level has the
 // rows to fill the chip (neighbouring rows' columns lie close together, so a warp's gathers touch
 // few sectors), else 2^lg lanes per row.
 template <bool SELL>
 static __global__ void __launch_bounds__(MLK_TPB) k_mlk_csweep(MlkLevel L, int step, int keep, float c1, float c2,
-                                                        const float* __restrict__ xi, float* __restrict__ xo,
+                                                        const float* xi, float* xo,
                                                         const MlkState* S) {
   mlk_enter();
   if (S->done) return;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const float acc = mlk_rowsum<SELL>(L.A, t, L.n, xi);
   const int i = mlk_row_of<SELL>(L.A, t, L.n);
-  if (i >= 0) mlk_step(L, step, keep, c1, c2, i, acc, __ldg(&xi[i]), xo, 0.0f);
+  if (i >= 0) mlk_step(L, step, keep, c1, c2, i, acc, mlk_ld(&xi[i]), xo, 0.0f);
 }
 // restriction P^T r: the next level's scaled right-hand side (or the coarsest one, unscaled)
 template <bool SELL>
-static __global__ void __launch_bounds__(MLK_TPB) k_mlk_restrict(MlkLevel L, const float* __restrict__ r, MlkLevel N,
-                                                          float* __restrict__ bC, const MlkState* S) {
+static __global__ void __launch_bounds__(MLK_TPB) k_mlk_restrict(MlkLevel L, const float* r, MlkLevel N,
+                                                          float* bC, const MlkState* S) {
   mlk_enter();
   if (S->done) return;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -311,8 +331,8 @@ static __global__ void __launch_bounds__(MLK_TPB) k_mlk_restrict(MlkLevel L, con
 }
 // coarsest level: x_C = A_C^-1 b_C, one warp per row; rows of the inverse and b_C padded with zeros
 // to a multiple of 4 (16-byte loads)
-static __global__ void __launch_bounds__(MLK_TPB) k_mlk_coarse(int nC, int nC4, const float4* __restrict__ cinv,
-                                                        const float4* __restrict__ bC, float* __restrict__ xC,
+static __global__ void __launch_bounds__(MLK_TPB) k_mlk_coarse(int nC, int nC4, const float4* cinv,
+                                                        const float4* bC, float* xC,
                                                         const MlkState* S) {
   mlk_enter();
   if (S->done) return;
@@ -323,7 +343,7 @@ static __global__ void __launch_bounds__(MLK_TPB) k_mlk_coarse(int nC, int nC4, 
   float s = 0.0f;
 #pragma unroll 4
   for (int k = lane; k < nC4; k += 32) {
-    const float4 c = __ldg(&q[k]), b = __ldg(&bC[k]);
+    const float4 c = __ldg(&q[k]), b = mlk_ld(&bC[k]);
     s = fmaf(c.x, b.x, s);
     s = fmaf(c.y, b.y, s);
     s = fmaf(c.z, b.z, s);
@@ -334,8 +354,8 @@ static __global__ void __launch_bounds__(MLK_TPB) k_mlk_coarse(int nC, int nC4, 
 }
 // prolongation in place: x_i += oc (P x_c)_i
 template <bool SELL>
-static __global__ void __launch_bounds__(MLK_TPB) k_mlk_prolong(MlkLevel L, float* __restrict__ x,
-                                                         const float* __restrict__ xc, const MlkState* S) {
+static __global__ void __launch_bounds__(MLK_TPB) k_mlk_prolong(MlkLevel L, float* x,
+                                                         const float* xc, const MlkState* S) {
   mlk_enter();
   if (S->done) return;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -345,7 +365,7 @@ static __global__ void __launch_bounds__(MLK_TPB) k_mlk_prolong(MlkLevel L, floa
 }
 
 // training-sample recording of the learned term (as in k_mlcg): every rec_stride-th iteration
-static __global__ void __launch_bounds__(MLK_TPB) k_mlk_record(MlArgs a, const float* __restrict__ z, const float* b0,
+static __global__ void __launch_bounds__(MLK_TPB) k_mlk_record(MlArgs a, const float* z, const float* b0,
                                                         const MlkState* S) {
   mlk_enter();
   if (S->done) return;
@@ -365,7 +385,7 @@ static __global__ void __launch_bounds__(MLK_TPB) k_mlk_record(MlArgs a, const f
 // sweeps; a grid-stride loop over ~32 rows per thread ran at half the bandwidth), per-block
 // partials folded by k_mlk_fold before the scalar kernel
 template <class ZT>
-static __global__ void __launch_bounds__(MLK_TPB) k_mlk_wz(MlArgs a, const ZT* __restrict__ z, double* part,
+static __global__ void __launch_bounds__(MLK_TPB) k_mlk_wz(MlArgs a, const ZT* z, double* part,
                                                     const MlkState* S) {
   mlk_enter();
   if (S->done) return;
@@ -392,7 +412,7 @@ static __global__ void __launch_bounds__(MLK_TPB) k_mlk_wz(MlArgs a, const ZT* _
 // the blocks' values (fixed order), forms the FCG scalars and applies the stopping rule (k_mlcg's,
 // after its reduce-and-gather).  The iteration counted here is the one k_mlk_update ends; the cap
 // stops the solve at the next rule (KSP_DIVERGED_ITS).
-static __global__ void __launch_bounds__(MLK_TPB) k_mlk_rule(int n, int nparts, const double* __restrict__ in,
+static __global__ void __launch_bounds__(MLK_TPB) k_mlk_rule(int n, int nparts, const double* in,
                                                       double* part, MlkState* S) {
   mlk_enter();
   if (S->done) return;
@@ -450,7 +470,7 @@ static __global__ void __launch_bounds__(MLK_TPB) k_mlk_rule(int n, int nparts, 
 // p = (z - m) + beta p, q = w + beta q, x += alpha p, r -= alpha q, then level 0's scaled
 // right-hand side
 template <class ZT>
-static __global__ void __launch_bounds__(MLK_TPB) k_mlk_update(MlArgs a, const ZT* __restrict__ z, MlkLevel L0,
+static __global__ void __launch_bounds__(MLK_TPB) k_mlk_update(MlArgs a, const ZT* z, MlkLevel L0,
                                                         const MlkState* S) {
   mlk_enter();
   if (S->done) return;

@@ -2,6 +2,9 @@
 
 * A block of a cluster may touch another block's shared memory only after a cluster barrier has shown
   that the other block runs.
+* Kernels launched with programmatic stream serialization are resident while the one before still
+  writes.  What an earlier kernel of the chain writes is not read by the non-coherent load, nor through
+  a __restrict__ pointer, from which the compiler may load before the wait.
 """
 import os
 import re
@@ -45,3 +48,19 @@ def test_cluster_blocks_meet_before_the_first_remote_access():
     # reached by every thread: outside any block of the kernel's body
     for at in (arrive, wait):
         assert code[:at].count("{") - code[:at].count("}") == 1
+
+
+def test_chained_kernels_read_written_data_behind_the_wait():
+    src = _source("mlkern.cuh")
+    # arrays of the set-up, which no kernel of the chain writes (q: matrix entries, rows of the inverse)
+    constant = {"L.col", "L.dinv", "L.diag", "L.g", "m.off", "m.ent", "om", "a.pinv", "q"}
+    loads = re.findall(r"__ldg\(&([\w.]+)", src)
+    assert src.count("__ldg(") == len(loads)
+    assert set(loads) <= constant, set(loads) - constant
+    kernels = [k for k in _bodies(src, r"__global__[^;{]*?k_mlk_\w+") if "mlk_enter();" in k[1]]
+    assert len(kernels) >= 10
+    for sig, body in kernels:
+        assert "__restrict__" not in sig, sig
+        assert body[1:].lstrip().startswith("mlk_enter();"), sig
+    for sig, _ in _bodies(src, r"__device__[^;{]*?mlk_(?:rowsum|row0|step|start|totals)"):
+        assert "__restrict__" not in sig, sig
