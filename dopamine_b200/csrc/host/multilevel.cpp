@@ -254,7 +254,11 @@ bool cholesky_lower(std::vector<double>& a, int n) {
   return true;
 }
 
-int dense_inverse(const Csr& A, bool nullsp, std::vector<float>& out) {
+// region: of every row, where the operator falls apart into several (null: one region); lift: of every
+// region, whether its constant is in the null space.  The rows of skip (null: none) are closed regions
+// on their own: their rows of the inverse are zero.
+int dense_inverse(const Csr& A, bool nullsp, std::vector<float>& out, const std::vector<int>* region = nullptr,
+                  const std::vector<char>* lift = nullptr, const std::vector<char>* skip = nullptr) {
   const int n = A.n;
   std::vector<double> a((size_t)n * n, 0.0);
   double tr = 0.0;
@@ -263,7 +267,21 @@ int dense_inverse(const Csr& A, bool nullsp, std::vector<float>& out) {
       a[(size_t)i * n + A.col[k]] += A.val[k];
       if (A.col[k] == i) tr += A.val[k];
     }
-  if (nullsp) {  // constant mode lifted to the mean diagonal: (A + s 1 1^T) 1 = (tr / n) 1
+  if (region) {  // every closed region's own constant, as below
+    std::vector<double> trr(lift->size(), 0.0);
+    std::vector<int> m(lift->size(), 0);
+    for (int i = 0; i < n; ++i) {
+      if ((*skip)[i]) a[(size_t)i * n + i] = 1.0;  // alone in its row
+      trr[(*region)[i]] += a[(size_t)i * n + i];
+      m[(*region)[i]]++;
+    }
+    for (int i = 0; i < n; ++i) {
+      const int c = (*region)[i];
+      if (!(*lift)[c] || (*skip)[i]) continue;
+      for (int j = 0; j < n; ++j)
+        if ((*region)[j] == c) a[(size_t)i * n + j] += trr[c] / ((double)m[c] * m[c]);
+    }
+  } else if (nullsp) {  // constant mode lifted to the mean diagonal: (A + s 1 1^T) 1 = (tr / n) 1
     const double s = tr / ((double)n * n);
     for (auto& x : a) x += s;
   }
@@ -291,6 +309,9 @@ int dense_inverse(const Csr& A, bool nullsp, std::vector<float>& out) {
       out[(size_t)i * n + j] = (float)s;
       out[(size_t)j * n + i] = (float)s;
     }
+  if (region)
+    for (int i = 0; i < n; ++i)
+      if ((*skip)[i]) out[(size_t)i * n + i] = 0.0f;
   return 0;
 }
 
@@ -608,10 +629,58 @@ int scaled_rows(const Csr& A, const std::vector<double>& dinv, bool ell, bool ha
         else L.sv32[e] = 0.0f;
       }
     L.g[i] = (float)d;
-    L.diag[i] = (float)(1.0 / dinv[i]);
+    L.diag[i] = dinv[i] > 0.0 ? (float)(1.0 / dinv[i]) : 0.0f;  // 0: a closed region on its own
     L.dinv[i] = (float)dinv[i];
   }
   return 0;
+}
+
+// A region whose sum of entries is this small a part of its diagonals is closed: no Dirichlet row holds
+// its constant.  The sums of closed regions are rounding (below 1e-15); one Dirichlet face on a region
+// of 10^7 cells is about 1e-8.
+constexpr double CLOSED = 1e-11;
+
+// Of every row of U = T^T A T: whether it is a closed region on its own; empty when no row is.  before:
+// the same of A's rows (their diagonals are rounding already).
+std::vector<char> closed_rows(const Csr& A, const Csr& U, const std::vector<int>& agg,
+                              const std::vector<char>& before) {
+  std::vector<char> closed;
+  auto alone = [](const Csr& C, int i) { return C.off[i + 1] - C.off[i] == 1; };
+  for (int c = 0; c < U.n; ++c)
+    if (alone(U, c) && closed.empty()) closed.assign(U.n, 0);
+  if (closed.empty()) return closed;
+  std::vector<double> dg(U.n, 0.0);
+  for (int i = 0; i < A.n; ++i)
+    for (int64_t k = A.off[i]; k < A.off[i + 1]; ++k)
+      if (A.col[k] == i) dg[agg[i]] += A.val[k];
+  for (int c = 0; c < U.n; ++c)
+    closed[c] = alone(U, c) && U.val[U.off[c]] <= CLOSED * dg[c];
+  for (size_t i = 0; i < before.size(); ++i)
+    if (before[i]) closed[agg[i]] = 1;
+  return closed;
+}
+
+// Regions of A that do not touch one another, numbered in order of their first row.
+int regions(const Csr& A, std::vector<int>& region) {
+  region.assign(A.n, -1);
+  int nr = 0;
+  std::vector<int> todo;
+  for (int r = 0; r < A.n; ++r) {
+    if (region[r] >= 0) continue;
+    region[r] = nr;
+    todo.assign(1, r);
+    while (!todo.empty()) {
+      const int i = todo.back();
+      todo.pop_back();
+      for (int64_t k = A.off[i]; k < A.off[i + 1]; ++k)
+        if (region[A.col[k]] < 0) {
+          region[A.col[k]] = nr;
+          todo.push_back(A.col[k]);
+        }
+    }
+    ++nr;
+  }
+  return nr;
 }
 
 }  // namespace
@@ -622,6 +691,9 @@ int build_smoothed_multilevel(int n, int WA, const int* A_col, const double* A_v
   if (n < 1 || WA < 1 || WA > 64 || passes < 1 || ncoarse < 1) return -1;
   M = SaMultilevel{};
   Csr A = csr_from_ell(n, WA, A_col, A_val), U;  // U: the unsmoothed Galerkin operator of this level
+  // Rows that are closed regions on their own (empty: none).  Such a row's constant is all it has, which no
+  // level can correct: its 1/diagonal is taken as zero.
+  std::vector<char> closed;
   for (;;) {
     const Csr& from = M.lv.empty() ? A : U;
     M.sizes.push_back(A.n);
@@ -641,6 +713,7 @@ int build_smoothed_multilevel(int n, int WA, const int* A_col, const double* A_v
           ++nd;
         }
       }
+      if (!closed.empty() && closed[i]) continue;
       if (!(dg > 0.0) || nd != 1) {
         bad = 1;
         continue;
@@ -687,12 +760,26 @@ int build_smoothed_multilevel(int n, int WA, const int* A_col, const double* A_v
       C = galerkin(A, agg, na);
     }
     L.n_next = na;
+    closed = closed_rows(from, Un, agg, closed);
     M.lv.push_back(std::move(L));
     A = std::move(C);
     U = std::move(Un);
   }
   M.nC = A.n;
-  return dense_inverse(A, nullsp, M.cinv);
+  const Csr& from = M.lv.empty() ? A : U;
+  std::vector<int> region;
+  const int nr = regions(from, region);
+  if (nr == 1) return dense_inverse(A, nullsp, M.cinv);
+  std::vector<double> sum(nr, 0.0), dg(nr, 0.0);
+  for (int i = 0; i < A.n; ++i)
+    for (int64_t k = from.off[i]; k < from.off[i + 1]; ++k) {
+      sum[region[i]] += from.val[k];
+      if (from.col[k] == i) dg[region[i]] += from.val[k];
+    }
+  std::vector<char> lift(nr);
+  for (int c = 0; c < nr; ++c) lift[c] = sum[c] <= CLOSED * dg[c];
+  closed.resize(A.n, 0);
+  return dense_inverse(A, nullsp, M.cinv, &region, &lift, &closed);
 }
 
 bool slice_rows(int rows, const Raw<int>& off, const Raw<SaEntry>& ent, Raw<int>& soff, Raw<SaEntry>& sent) {

@@ -107,6 +107,9 @@ struct SaMultilevel {
 // one more); with fewer than three, or where the smoothed Galerkin operator would hold more
 // entries than the level itself, the transfer stays unsmoothed with the over-correction oc.
 // half: the finest level's off-diagonals in binary16.  Coarsening stops at <= ncoarse rows.
+// Fluid regions that do not touch one another and hold no Dirichlet row each have their own constant in the
+// null space: the dense inverse lifts every one of them, and a region that has shrunk to one row gets no
+// coarse correction (its 1/diagonal and its row of the inverse are zero).
 int build_smoothed_multilevel(int n, int WA, const int* A_col, const double* A_val, bool nullsp, int passes,
                               double beta, double oc, bool half, int ncoarse, SaMultilevel& M);
 
