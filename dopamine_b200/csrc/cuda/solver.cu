@@ -602,9 +602,19 @@ struct Solver {
       // cost 14-27 us and their number grows with the mesh.  Poisson ms per step, two-level and
       // multilevel: 108 000 cells 3.5 / 3.7 and 5.7 / 5.9, 148 640 cells 6.9 / 6.5, 175 616 cells
       // 4.5 / 3.5, 393 216 cells 9.6 / 6.6.
-      int rc = nc <= AUTO_TWOLEVEL_CELLS && (nc + dev_sms - 1) / dev_sms <= 4096 ? setup_fcg(dev_sms)
-                                                                                 : DPM_ERR_UNSUPPORTED;
-      if (rc == DPM_ERR_UNSUPPORTED) rc = setup_ml(dev_sms);
+      // Beyond the limit the two-level form stays the one for operators that the multilevel set-up refuses.
+      const bool fits = (nc + dev_sms - 1) / dev_sms <= 4096, first = fits && nc <= AUTO_TWOLEVEL_CELLS;
+      int rc = first ? setup_fcg(dev_sms) : DPM_ERR_UNSUPPORTED;
+      if (rc == DPM_ERR_UNSUPPORTED) {
+        float theta, delta;
+        if (fits && !first && smoother_interval(&theta, &delta)) return DPM_ERR_ARG;  // as the two-level form refuses it
+        rc = setup_ml(dev_sms);
+        if (rc && rc != DPM_ERR_CUDA && fits && !first) {
+          ml.release();
+          const int rc2 = setup_fcg(dev_sms);
+          if (rc2 != DPM_ERR_UNSUPPORTED) rc = rc2;
+        }
+      }
       if (rc) return rc;
     } else if (P.p_solver != DPM_PSOLVER_JACOBI_PCG) {
       return DPM_ERR_ARG;
@@ -1121,6 +1131,16 @@ struct Solver {
     }
   }
 
+  // Centre and half width of the two-level form's Chebyshev interval.
+  int smoother_interval(float* theta, float* delta) const {
+    const double lmin = P.p_smooth_lmin > 0.0 ? P.p_smooth_lmin : 0.05;
+    const double lmax = P.p_smooth_lmax > 0.0 ? P.p_smooth_lmax : 2.0;
+    if (!(lmax > lmin)) return DPM_ERR_ARG;
+    *theta = (float)(0.5 * (lmax + lmin));
+    *delta = (float)(0.5 * (lmax - lmin));
+    return 0;
+  }
+
   // Two-level FCG set-up: one part per SM (the kernel needs one co-resident block per part and
   // its part's local operator in shared memory).
   int setup_fcg(int dev_sms) {
@@ -1163,11 +1183,7 @@ struct Solver {
     fa.bar = cg_bar; fa.status = cg_status; fa.dout = cg_dout;
     fa.nullsp = nullsp ? 1 : 0;
     fa.degree = P.p_smooth_degree > 0 ? P.p_smooth_degree : 7;
-    const double lmin = P.p_smooth_lmin > 0.0 ? P.p_smooth_lmin : 0.05;
-    const double lmax = P.p_smooth_lmax > 0.0 ? P.p_smooth_lmax : 2.0;
-    if (!(lmax > lmin)) return DPM_ERR_ARG;
-    fa.theta = (float)(0.5 * (lmax + lmin));
-    fa.delta = (float)(0.5 * (lmax - lmin));
+    if (smoother_interval(&fa.theta, &fa.delta)) return DPM_ERR_ARG;
     fcg_WA = T.WA;
     if (!fa.partials || !fa.zs) return DPM_ERR_CUDA;
     fa.stall_window = P.p_stall_window > 0 ? P.p_stall_window : 50;
