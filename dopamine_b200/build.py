@@ -20,7 +20,7 @@ CU_FLAGS = {"csrc/cuda/setup_gpu.cu": ["-fmad=false"]}
 CPP_SOURCES = ["csrc/host/mesh.cpp", "csrc/host/ops.cpp", "csrc/host/twolevel.cpp", "csrc/host/multilevel.cpp",
                "csrc/host/gmsh.cpp", "csrc/host/foam.cpp"]
 HEADERS = ["csrc/cuda/common.cuh", "csrc/cuda/kernels.cuh", "csrc/cuda/pcg.cuh", "csrc/cuda/pcg_cluster.cuh", "csrc/cuda/fcg.cuh",
-           "csrc/cuda/learn.cuh", "csrc/cuda/scalars.cuh", "csrc/cuda/mlcg.cuh", "csrc/cuda/mlsolve.cuh", "csrc/cuda/mlkern.cuh", "csrc/cuda/explicit32.cuh",
+           "csrc/cuda/learn.cuh", "csrc/cuda/scalars.cuh", "csrc/cuda/mlcg.cuh", "csrc/cuda/mlsolve.cuh", "csrc/cuda/mlkern.cuh", "csrc/cuda/capture.hpp", "csrc/cuda/explicit32.cuh",
            "csrc/cuda/setup_gpu.hpp", "csrc/cuda/cellproj.cuh", "csrc/cuda/sampling.cuh", "csrc/cuda/forcing.cuh", "csrc/cuda/sem.cuh", "csrc/host/fortran_records.hpp",
            "csrc/host/twolevel.hpp", "csrc/host/multilevel.hpp", "csrc/host/mesh.hpp", "csrc/host/gmsh.hpp",
            "csrc/host/ops.hpp", "../include/dopamine_b200.h"]

@@ -10,6 +10,7 @@
 
 #include "../../../include/dopamine_b200.h"
 #include "../host/multilevel.hpp"
+#include "capture.hpp"
 #include "mlcg.cuh"
 #include "mlkern.cuh"
 
@@ -375,18 +376,7 @@ struct MlSolver {
   cudaGraphExec_t iteration_graph(const MlArgs& a, cudaStream_t st) {
     if (gexec && gexec_gamma == a.gamma && gexec_omega == a.omega) return gexec;
     drop_graph();
-    cudaGraph_t g = nullptr;
-    if (cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) != cudaSuccess) return nullptr;
-    enqueue_iteration(a, st);
-    if (cudaStreamEndCapture(st, &g) != cudaSuccess || !g) {
-      cudaGetLastError();
-      return nullptr;
-    }
-    if (cudaGraphInstantiate(&gexec, g, 0) != cudaSuccess) {
-      cudaGetLastError();
-      gexec = nullptr;
-    }
-    cudaGraphDestroy(g);
+    gexec = capture_graph(st, [&] { enqueue_iteration(a, st); });
     gexec_gamma = a.gamma;
     gexec_omega = a.omega;
     return gexec;
