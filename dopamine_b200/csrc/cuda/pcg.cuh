@@ -400,26 +400,26 @@ struct PcgScalars {
   }
 };
 
-// Staged form: block b owns the consecutive rows [b C, b C + size) and keeps the operator (the first
-// WS slots of its rows) and its part of p in shared memory, x, r, p, q and 1/diag in registers.  The
+// Staged form: block b owns the consecutive rows [b C, b C + size) and keeps their operator (200 B per
+// row of 16, the widest) and its part of p in shared memory, x, r, p, q and 1/diag in registers.  The
 // entries of a row that lie in the block's own rows - five of seven on a hexahedral mesh - read p
 // there; the others form p_j from z_j and the old p_j in L2, as k_pcg does for all.
-// us per iteration, here and in the form that reads all of it through L2: 44 880 rows 6.8 / 8.8,
-// 66 600 rows 6.9 / 8.85, 85 050 rows 7.5 / 8.9.  With more than two rows per thread the few warps no
+// us per iteration (of two solves that differ by 100), here and in the form that reads all of it through
+// L2: 44 880 rows 6.0 / 8.45, 66 600 rows 6.1 / 8.5, 85 050 rows 6.6 / 8.6, 131 072 rows 6.7 / 8.8.  With more than two rows per thread the few warps no
 // longer cover the loads from other blocks' rows, one row after the other (393 216 rows, six rows per
 // thread: 15.5 / 12.7), and the register form with 32 warps takes over.
 // CPT: rows per thread.
 constexpr int PCG_ST_TPB = 512;
 constexpr int PCG_ST_CPT = 2;
 template <int CPT, int WT>
-__global__ void __launch_bounds__(PCG_ST_TPB, 1) k_pcg_staged(PcgArgs<double> a, int C, int WC, int WS) {
+__global__ void __launch_bounds__(PCG_ST_TPB, 1) k_pcg_staged(PcgArgs<double> a, int C) {
   extern __shared__ double st_smem[];
   constexpr int CH = WT > 0 ? WT : 4;  // slots whose loads are in flight together
   const int n = a.n, WA = WT > 0 ? WT : a.WA;
   const int base = (int)blockIdx.x * C, size = max(0, min(C, n - base));
   double* s_p = st_smem;                               // [C]
-  double* s_val = s_p + C;                             // [WS][C]
-  int* s_col = reinterpret_cast<int*>(s_val + (size_t)WS * C);  // [WC][C] own row l, or ~global column
+  double* s_val = s_p + C;                             // [WA][C]
+  int* s_col = reinterpret_cast<int*>(s_val + (size_t)WA * C);  // [WA][C] own row l, or ~global column
   unsigned gen = 0;
   auto code = [&](int c) { return (unsigned)(c - base) < (unsigned)size ? c - base : ~c; };
   // row l of this block times the vector that is s_p on its own rows and elsewhere z - m + f po (no f:
@@ -433,8 +433,8 @@ __global__ void __launch_bounds__(PCG_ST_TPB, 1) k_pcg_staged(PcgArgs<double> a,
       for (int u = 0; u < CH; ++u) {
         const int w = w0 + u;
         const bool on = WT > 0 || w < WA;
-        cc[u] = !on ? l : w < WC ? s_col[w * C + l] : code(__ldg(&a.col[(size_t)w * n + base + l]));
-        v[u] = !on ? 0.0 : w < WS ? s_val[w * C + l] : __ldcg(&a.val[(size_t)w * n + base + l]);
+        cc[u] = on ? s_col[w * C + l] : l;
+        v[u] = on ? s_val[w * C + l] : 0.0;
       }
       double zz[CH], pp[CH];
 #pragma unroll
@@ -458,10 +458,10 @@ __global__ void __launch_bounds__(PCG_ST_TPB, 1) k_pcg_staged(PcgArgs<double> a,
   };
 #define ST_OWN(k) ((int)threadIdx.x + (k) * PCG_ST_TPB < size)
 #define ST_ROW(k) ((int)threadIdx.x + (k) * PCG_ST_TPB)
-  for (int w = 0; w < WC; ++w)
+  for (int w = 0; w < WA; ++w)
     for (int l = threadIdx.x; l < size; l += PCG_ST_TPB) {
       s_col[w * C + l] = code(__ldg(&a.col[(size_t)w * n + base + l]));
-      if (w < WS) s_val[w * C + l] = __ldg(&a.val[(size_t)w * n + base + l]);
+      s_val[w * C + l] = __ldg(&a.val[(size_t)w * n + base + l]);
     }
   double rx[CPT], rr[CPT], rp[CPT], rq[CPT], rd[CPT];
   // ---- b' = b - mean(b) when the constant null space is active; the guess
@@ -589,12 +589,15 @@ __global__ void __launch_bounds__(PCG_ST_TPB, 1) k_pcg_staged(PcgArgs<double> a,
 #undef ST_ROW
 }
 
-// The cooperative launch of a system: kernel, blocks, rows per block, staged slots, shared memory.
+constexpr size_t pcg_staged_smem(int rows, int width) { return (size_t)rows * (8 + 12 * (size_t)width); }
+
+// The cooperative launch of a system: kernel, blocks, rows per block, shared memory.
 struct PcgGrid {
   void* kernel = nullptr;
-  int grid = 0, tpb = 0, C = 0, WC = 0, WS = 0;  // WC, WS: slots whose columns and values are staged
+  int grid = 0, tpb = 0, C = 0;
   size_t smem = 0;
   static constexpr int max_smem = 223 * 1024;  // of 227 KB per block; the all-reduces' buffers take 3 KB
+  static_assert(pcg_staged_smem(PCG_ST_TPB * PCG_ST_CPT, 16) <= max_smem, "the widest operator is staged whole");
 
   template <int CPT>
   static void* pick_cpt(int cpt, int width) {
@@ -625,14 +628,7 @@ struct PcgGrid {
     const int cpt = (C + PCG_ST_TPB - 1) / PCG_ST_TPB;
     const bool st = cpt <= PCG_ST_CPT;
     tpb = st ? PCG_ST_TPB : PCG_TPB;
-    WC = WS = 0;
-    smem = 0;
-    if (st) {  // columns first: a column from L2 delays the load that depends on it
-      const size_t words = max_smem / (4 * (size_t)C) - 2;
-      WC = (int)std::min<size_t>(width, words);
-      WS = (int)std::min<size_t>(WC, (words - WC) / 2);
-      smem = 4 * (size_t)C * (2 + WC + 2 * WS);
-    }
+    smem = st ? pcg_staged_smem(C, width) : 0;
     const int rows = (C + PCG_TPB - 1) / PCG_TPB;  // of a thread in the register form
     void* k = st ? staged(cpt, width) : regs(rows >= 2 && rows <= 4 ? rows : 0, width);
     int per_sm = 0;
@@ -643,8 +639,8 @@ struct PcgGrid {
     return true;
   }
   cudaError_t launch(PcgArgs<double> a, cudaStream_t st) const {
-    int rows = C, cols = WC, slots = WS;
-    void* staged_args[] = {&a, &rows, &cols, &slots};
+    int rows = C;
+    void* staged_args[] = {&a, &rows};
     return cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(tpb), staged_args, smem, st);  // k_pcg takes the first
   }
 };
