@@ -127,8 +127,9 @@ def test_dropin_boomeramg_name_selects_the_multilevel_solve():
 
 
 def test_auto_picks_the_form_that_fits():
-    """p_solver = DPM_PSOLVER_AUTO takes the two-level form while the mesh has at most 4096 cells
-    per SM and the multilevel form beyond; the stats report the form in use."""
+    """p_solver = DPM_PSOLVER_AUTO takes the two-level form on a small mesh and the multilevel form on one of
+    786 432 cells, which the two-level kernel could not hold (4096 cells per SM); the stats report the form
+    in use.  test_gpu_auto_form.py has the limit between them."""
     small = cases.channel_config(nx=16, ny=12, nz=8, n_steps=1)
     p = small.make_params()
     p.p_solver = abi.PSOLVER_AUTO

@@ -73,3 +73,56 @@ def test_step_operators_match_plain_pcg(name):
     U, st = _step(case, p_solver=abi.PSOLVER_MULTILEVEL_FCG)
     assert st["p_fallbacks"] == 0 and st["p_iters"] <= 30 * st["p_solves"], st
     assert np.linalg.norm(U - U0) <= 1e-8 * np.linalg.norm(U0)
+
+
+def _fields(case, steps=2, **kw):
+    s = Solver(case, params=abi.default_params(**dict(case.params, **kw)))
+    s.initialise()
+    for _ in range(steps):
+        s.advance()
+    h, st = s.sync_host(), s.stats()
+    out = {"U": h["U"], "p": h["p"] - h["p"].mean()}
+    if s.params.sgs_model != abi.SGS_NONE:
+        out["nu_sgs"] = h["nu_sgs"]
+    if s.params.boussinesq:
+        out["T"] = h["T"]
+    if s.params.n_scalars:
+        out["C"] = s.scalars()[1]
+    s.close()
+    return out, st
+
+
+@pytest.mark.parametrize("flow", ["channel", "rb"])
+def test_every_field_matches_plain_pcg(flow):
+    """U, p, nu_sgs, T and the scalars after two steps.  Both forms stop at ||r|| <= 1e-12 ||b||: with a
+    condition number below 1e5 the pressures differ by less than 1e-7 and what they correct by less."""
+    case = (cases.channel_config(nx=60, ny=37, nz=33, n_steps=2) if flow == "channel" else
+            cases.rb_config(nx=48, ny=48, nz=33))
+    ref, _ = _fields(case, p_tol=1e-12)
+    out, st = _fields(case, p_tol=1e-12, p_solver=abi.PSOLVER_MULTILEVEL_FCG)
+    assert st["p_fallbacks"] == 0
+    err = {k: np.linalg.norm(out[k] - ref[k]) / np.linalg.norm(ref[k]) for k in ref}
+    print(flow, {k: f"{v:.1e}" for k, v in err.items()})
+    assert err.pop("p") <= 1e-7, err
+    assert max(err.values()) <= 1e-8, err
+
+
+def test_every_field_of_the_urban_flow():
+    """At single near-ground cells the surface flux amplifies the last bits of the solve, whatever solves: plain
+    PCG at p_tol 1e-10 against itself at 1e-13 moves U by 3.1e-6 (8.9e-6 on 60x60x19), p by 1.1e-4 (6.9e-4),
+    nu_sgs by 2.5e-5 and the scalar by 1.1e-5 relative.  About four times that is allowed."""
+    case = cases.urban_config(100, 100, 32)
+    ref, _ = _fields(case, p_tol=1e-13)
+    out, st = _fields(case, p_tol=1e-13, p_solver=abi.PSOLVER_MULTILEVEL_FCG)
+    assert st["p_fallbacks"] == 0
+    err = {k: np.linalg.norm(out[k] - ref[k]) / np.linalg.norm(ref[k]) for k in ref}
+    print("urban", {k: f"{v:.1e}" for k, v in err.items()})
+    for k, tol in {"U": 3.6e-5, "p": 2.8e-3, "nu_sgs": 1e-4, "C": 4.4e-5, "T": 1e-5}.items():
+        assert err[k] <= tol, (k, err)
+
+
+def test_solve_repeats_bit_for_bit():
+    case = cases.urban_config(100, 100, 32)
+    a, _ = _fields(case, steps=1, p_solver=abi.PSOLVER_MULTILEVEL_FCG)
+    b, _ = _fields(case, steps=1, p_solver=abi.PSOLVER_MULTILEVEL_FCG)
+    assert all(np.array_equal(a[k], b[k]) for k in a)
