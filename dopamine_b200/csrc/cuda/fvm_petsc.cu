@@ -3,8 +3,10 @@
 // Same symbols, arguments and status codes as the PETSc backend.  The preconditioner names of
 // fvm_petsc_set_pressure_solver select the Krylov kernel: "boomeramg" and "gamg" (the
 // reference's algebraic-multigrid choices, pressure_backend_petsc.c:10, :533-537) run flexible CG
-// with the FP32 aggregation-multigrid V-cycle of mlcg.cuh; "jacobi" (or -pc_type jacobi through
-// fvm_petsc_insert_option), and the state before any selection, run the Jacobi-PCG of pcg.cuh.
+// with the FP32 smoothed-aggregation V-cycle of mlkern.cuh (the unsmoothed one of mlcg.cuh up to 1200
+// rows and where the smoothed set-up refuses the operator); "jacobi" (or -pc_type jacobi through
+// fvm_petsc_insert_option), and the state before any selection, run the Jacobi-PCG of pcg_cluster.cuh
+// (up to 40 960 rows) and pcg.cuh.
 // Conventions kept from the reference:
 //  * indices are 1-based, face_neighbor_global <= 0 or skip_face != 0 drops a face;
 //  * the operator is assembled once and cached; it is rebuilt when n_cells, n_faces or the

@@ -12,7 +12,8 @@
 // The Krylov state lives in device memory (MlkState); once a solve has stopped, every kernel returns
 // at its first instruction, so the host enqueues the next iteration before it reads the stop flag of
 // the last one.  An iteration is one captured graph whose kernels follow each other with
-// programmatic launches (mlk_enter): 27 launches of 3-60 us each had left 4-5 us between them.
+// programmatic launches (mlk_enter): single launches of 3-60 us each had left 4-5 us between them.  At
+// Chebyshev degree 2 an iteration of L smoothed levels is 6 L + 4 launches: 16, 22 or 28.
 //
 // The hierarchy is smoothed aggregation (SaLevel, csrc/host/multilevel.hpp).  The unsmoothed one of
 // k_mlcg moves a quarter fewer bytes per iteration, but its two-grid contraction is 0.4-0.5 whatever
@@ -20,10 +21,11 @@
 // operator), against 0.17-0.36 here: 12 iterations per solve instead of 31 there (Poisson 45.1 ->
 // 18.0 ms per step), 13.7 instead of 36 at 8.2M cells (127 -> 57 ms), 22 instead of 29 on the
 // graded 1.06M-cell Rayleigh-Benard mesh (24.7 -> 14.3 ms).
-// Bounds: the finest level's sweeps and the FP64 passes stream at the copy bandwidth (72 B per row
-// and sweep, 26 us for 2.4M rows); the first coarse level's rows (37 entries) are bound by their
-// gathers, so they are laid out as slices with a row per thread: 22 us per sweep of 304k rows, 41
-// with eight lanes per row; levels below ~20k rows cost their launch and latency, 4-10 us.
+// Bounds (ncu, 2.4M rows): the finest level's sweeps stream 68 B per row, 33 us at 5.0 of the 6.47 TB/s
+// a copy reaches, the FP64 w = A z 4.0 and the update 5.4 TB/s; the first coarse level's rows (37 entries)
+// are bound by the latency of their gathers, 28 us per sweep of 304k rows at 3.8 TB/s: they are laid out
+// as slices with a row per thread (22 us when the two were compared, 41 with eight lanes per row); levels
+// below ~20k rows cost their launch and latency, 4-10 us.
 // The recurrences, the null-space handling, the stall guard and the stopping rule are those of
 // k_mlcg and k_fcg (src/solver/pressure_backend_petsc.c:816-876 for the rule itself); only the
 // order of the reductions' sums differs.
@@ -134,7 +136,7 @@ struct MlkLevel {
 };
 
 // The scaled right-hand side of level L.  The first Chebyshev step from a zero iterate is
-// x = d = inv_theta b: it is not stored, mlk_cheb forms it from b (deg > 1) or k_mlk_first writes it.
+// x = d = inv_theta b: it is not stored, the sweep of STEP_SECOND forms it from b (deg > 1) or k_mlk_first writes it.
 __device__ __forceinline__ void mlk_start(const MlkLevel& L, int i, float ri) { L.b[i] = ri * __ldg(&L.dinv[i]); }
 
 // A smoothing step of one row.  STEP_SECOND: the second step from a zero iterate (the gathered
@@ -383,7 +385,7 @@ static __global__ void __launch_bounds__(MLK_TPB) k_mlk_record(MlArgs a, const f
 
 // ---- w = A z (FP64 operator) and the eight sums of the iteration: one row per thread (as the
 // sweeps; a grid-stride loop over ~32 rows per thread ran at half the bandwidth), per-block
-// partials folded by k_mlk_fold before the scalar kernel
+// partials folded by k_mlk_rule
 template <class ZT>
 static __global__ void __launch_bounds__(MLK_TPB) k_mlk_wz(MlArgs a, const ZT* z, double* part,
                                                     const MlkState* S) {

@@ -1,5 +1,6 @@
-// Host side of the multilevel flexible-CG solve (k_mlcg), shared by the solver object and the
-// drop-in pressure ABI: builds the hierarchy (csrc/host/multilevel.cpp), uploads the FP32 levels, sets the Chebyshev coefficients, sizes the cooperative grid and launches.
+// Host side of the multilevel flexible-CG solve, shared by the solver object and the drop-in pressure
+// ABI: builds the hierarchy (csrc/host/multilevel.cpp), uploads the FP32 levels, sets the Chebyshev
+// coefficients, and launches either the persistent kernel (k_mlcg) or the standalone ones (k_mlk_*).
 #pragma once
 #include <cuda_runtime.h>
 
@@ -26,10 +27,11 @@ struct MlSolver {
   // Multi-kernel form (mlkern.cuh) for fine levels of at least kernels_min_rows rows: the smoothed-
   // aggregation levels on the host for by-value launches, the Krylov state, partial sums, a
   // residual scratch vector, and two pinned stop flags with their events, used in turn.
-  // Rows from which a solver handle uses it (the drop-in solve does at any size).  It is the faster
-  // one everywhere: 32 768 rows 2.1 against 5.9 ms of Poisson solve per step, 299 764 rows 4.6
-  // against 10.7, 737 280 rows 8 against 22.6.  Smaller handles keep the persistent kernel, whose
-  // grid-wide waits dpm_set_barrier_spin_limit bounds and reports.
+  // Rows from which a solver handle uses it (the drop-in solve does from 1201).  It is the faster one at
+  // every size measured: 32 768 rows 2.1 against 5.9 ms of Poisson solve per step, 299 764 rows 4.6
+  // against 10.7, 737 280 rows 8 against 22.6.  The line is not where the times cross: handles below it,
+  // which the automatic choice gives the two-level form, keep the persistent kernel, whose grid-wide waits
+  // dpm_set_barrier_spin_limit bounds and reports; these kernels have no such waits.
   static constexpr int kernels_min_rows = 1 << 16;
   bool multi = false;
   double bytes_per_iteration = 0.0;  // algorithmic bytes of one Krylov iteration (roofline numerator)

@@ -11,8 +11,8 @@
 // which forms its neighbours' p from z and the old p): half the bytes gathered from shared memory,
 // which bound the kernel at 2000 rows per block and more.  Microseconds per iteration, here and
 // k_pcg: 1000 rows 3.5 / 9.4, 9216 rows 4.0 / 8.9, 32 768 rows 4.9 / 8.8, 35 937 rows 5.7 / 8.9;
-// beyond 40 960 rows the operator no longer fits the cluster's shared memory (44 880 rows 8.2 / 8.8,
-// 50 400 rows 10.6 / 8.8).
+// beyond 40 960 rows more of the operator than its last slot would have to come from L2 (44 880 rows
+// 8.2 / 8.8, 50 400 rows 10.6 / 8.8).
 //
 // Its waits need no poll limit: the blocks of a cluster are scheduled together, and every thread
 // reaches every barrier.  Scheduled together does not mean started: a block's shared memory may be

@@ -734,8 +734,8 @@ int build_smoothed_multilevel(int n, int WA, const int* A_col, const double* A_v
     int np = passes;
     if (!M.lv.empty()) {
       np = passes + 1;
-      // a coarsening that can reach the dense level does: on a 300 000-cell mesh 15 iterations of 15
-      // launches instead of 13 of 21, when every launch on the coarse levels costs its latency
+      // a coarsening that can reach the dense level does: on a 300 000-cell mesh 15 iterations of 16
+      // launches instead of 13 of 22, when every launch on the coarse levels costs its latency
       if (A.n <= 32 * ncoarse)
         for (np = 1; np < 5 && (A.n >> np) > ncoarse;) ++np;
     }

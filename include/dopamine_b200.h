@@ -445,7 +445,9 @@ int dpm_select_pressure_solver(dpm_solver_t* s, int p_solver);
  * `spins` polls of its arrival counter (0 restores the default, 2^26 polls, about a second).  A
  * wait that runs out sets the kernel's status word, every block returns, and the call that
  * launched it returns DPM_ERR_BARRIER_TIMEOUT; the handle stays usable.  Tests use a tiny value
- * to exercise that path without hanging or faulting the GPU. */
+ * to exercise that path without hanging or faulting the GPU.  While a limit is set, small Jacobi-PCG
+ * solves run the grid form instead of the cluster form; the multilevel form's kernels for meshes of
+ * 65 536 cells and more have no grid-wide waits. */
 int dpm_set_barrier_spin_limit(dpm_solver_t* s, long long spins);
 
 /* ---------------------------------------------------------------------------------------- */
