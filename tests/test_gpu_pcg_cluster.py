@@ -1,5 +1,5 @@
 """Jacobi-PCG on one thread-block cluster (pcg_cluster.cuh) at the edges of its range: one row, one
-block, sizes that leave the last block short or empty, one to five rows per thread, the largest
+block, sizes that leave the last block short, one to five rows per thread, the largest
 system it takes and the first it does not, rows wider and narrower than seven, operators that stay in
 shared memory and ones that do not fit, a non-zero guess, and the iteration cap.
 
