@@ -599,9 +599,16 @@ struct Solver {
       if (rc) return rc;
     } else if (P.p_solver == DPM_PSOLVER_AUTO) {
       // The two-level kernel keeps a part of <= 4096 cells per block, one block per SM; its iterations
-      // cost 14-27 us and their number grows with the mesh.  Poisson ms per step, two-level and
-      // multilevel: 108 000 cells 3.5 / 3.7 and 5.7 / 5.9, 148 640 cells 6.9 / 6.5, 175 616 cells
-      // 4.5 / 3.5, 393 216 cells 9.6 / 6.6.
+      // cost 14-27 us and their number grows with the mesh and its anisotropy.  ms per step, two-level and
+      // multilevel, precision form:
+      //   channel  135 168 cells 8.3 / 5.1    145 200  6.0 / 5.7    165 888  7.4 / 7.0    196 608 11.0 / 6.5
+      //   box      127 514 cells 8.9 / 8.0    148 640  9.2 / 8.3    199 268 11.3 / 10.4
+      //   urban    181 717 cells 6.0 / 5.6    299 764  7.4 / 7.3
+      //   RB       122 880 cells 5.2 / 5.5    135 168  5.8 / 6.8    156 816  7.2 / 6.6    186 624  7.4 / 7.6
+      //            230 400 cells 7.4 / 7.1    368 640  9.8 / 10.2
+      // No line in the number of cells serves all of them: Rayleigh-Benard meshes just above it, graded
+      // and of odd layers, take 23-25 multilevel iterations instead of 17-21 and lose up to 18 %, where
+      // channels gain up to 1.7x.
       // Beyond the limit the two-level form stays the one for operators that the multilevel set-up refuses.
       const bool fits = (nc + dev_sms - 1) / dev_sms <= 4096, first = fits && nc <= AUTO_TWOLEVEL_CELLS;
       int rc = first ? setup_fcg(dev_sms) : DPM_ERR_UNSUPPORTED;

@@ -69,7 +69,7 @@ extern "C" {
 #define DPM_PSOLVER_JACOBI_PCG 0
 #define DPM_PSOLVER_TWOLEVEL_FCG 1
 #define DPM_PSOLVER_MULTILEVEL_FCG 2  /* FCG + FP32 aggregation-multigrid V-cycle (no reference counterpart) */
-#define DPM_PSOLVER_AUTO 3  /* the faster one: two-level up to 131 072 cells (where the mesh fits it, <= 4096 cells per SM), else multilevel; two-level beyond where it fits and the multilevel set-up refuses the operator */
+#define DPM_PSOLVER_AUTO 3  /* by size: two-level up to 131 072 cells (where the mesh fits it, <= 4096 cells per SM), else multilevel; two-level beyond where it fits and the multilevel set-up refuses the operator */
 #define DPM_GRAD_LEAST_SQUARES 0
 #define DPM_GRAD_GREEN_GAUSS 1
 #define DPM_CELL_PROJECTION_LS 0
