@@ -405,9 +405,10 @@ struct PcgScalars {
 // entries of a row that lie in the block's own rows - five of seven on a hexahedral mesh - read p
 // there; the others form p_j from z_j and the old p_j in L2, as k_pcg does for all.
 // us per iteration (of two solves that differ by 100), here and in the form that reads all of it through
-// L2: 44 880 rows 6.0 / 8.45, 66 600 rows 6.1 / 8.5, 85 050 rows 6.6 / 8.6, 131 072 rows 6.7 / 8.8.  With more than two rows per thread the few warps no
-// longer cover the loads from other blocks' rows, one row after the other (393 216 rows, six rows per
-// thread: 15.5 / 12.7), and the register form with 32 warps takes over.
+// L2: 44 880 rows 6.0 / 8.45, 66 600 rows 6.1 / 8.5, 85 050 rows 6.6 / 8.6, 131 072 rows 6.7 / 8.8.
+// With more than two rows per thread the few warps no longer cover the loads from other blocks' rows, one
+// row after the other (393 216 rows, six rows per thread: 15.5 / 12.7), and the register form with 32 warps
+// takes over.
 // CPT: rows per thread.
 constexpr int PCG_ST_TPB = 512;
 constexpr int PCG_ST_CPT = 2;
